@@ -91,8 +91,10 @@ typedef struct tfs_stats {
                                    1 software-pipelined                        */
     int32_t  sell_width;        /* uniform SELL-32 slice width, 0 if per slice  */
     int32_t  dic_kernel;        /* DIC application last launched: 0 level
-                                   kernels, 1 one-block (TFS_OPT_DIC_BLOCK)    */
-    int32_t  pad;
+                                   kernels or tiles, 1 one-block
+                                   (TFS_OPT_DIC_BLOCK)                         */
+    int32_t  dic_tiles;         /* tiles of the DIC application last launched
+                                   (TFS_OPT_DIC_TILES), 0 if not tiled         */
 } tfs_stats;
 
 /* ---- topology ----------------------------------------------------------- */
@@ -165,6 +167,12 @@ int tfs_set_default_precision(int mode);
                                     access window of the solve kernels (a
                                     limit of the calling process's context;
                                     default); 0 none                           */
+#define TFS_OPT_DIC_TILES    16  /* 1 DIC sweeps tile by tile, each tile with the
+                                    rows it depends on in one block's shared
+                                    memory, where the cell numbering keeps those
+                                    few (default; not where TFS_OPT_TAIL_PF,
+                                    _FWD_PRE or _BWD_PRE are 0); 0 the level
+                                    kernels                                     */
 
 /* One DIC application (the tfs_time_prec workload: factor from val, r = 1)
  * with its level launches stamped on the device: for slot k (launch order)

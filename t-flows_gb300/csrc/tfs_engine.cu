@@ -16,6 +16,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <tuple>
 #include <vector>
 
@@ -24,8 +25,26 @@
 #include "tfs_mixed.cuh"
 #include "tfs_spmv.cuh"
 #include "tfs_dic_block.cuh"
+#include "tfs_dic_tiles.cuh"
 
 using namespace tfs;
+
+// The tiled DIC's plan (tfs_dic_tiles_plan.h) of one arithmetic on the device.
+struct TileStore {
+    int tiles = 0;                       // 0: no plan, the level kernels sweep
+    int max_slots = 0, max_rounds = 0, max_lists = 0, ring_bytes = 0, smem_bytes = 0;
+    struct Dir {
+        TileRound *rounds = nullptr;
+        int *tile_round = nullptr, *vbeg = nullptr;
+        uint32_t *rows = nullptr;
+        unsigned char *packed = nullptr;
+        int *tile_list = nullptr;
+        uint8_t *lists = nullptr;
+        uint32_t *list_row = nullptr;
+        uint16_t *list_slot = nullptr;
+        int n_rounds = 0;
+    } dir[2];
+};
 
 // ------------------------------------------------------------ errors
 
@@ -435,6 +454,19 @@ static void rcm_order(int n, const std::vector<int> &row0, const std::vector<int
     for (int k = 0; k < n; k++) rcm_pos[order[k]] = k;
 }
 
+static void free_tiles(tfs_handle *h)
+{
+    for (TileStore *&S : h->tiles) {
+        if (!S) continue;
+        for (TileStore::Dir &D : S->dir)
+            for (void *p : {(void *)D.rounds, (void *)D.tile_round, (void *)D.vbeg, (void *)D.rows, (void *)D.packed,
+                            (void *)D.tile_list, (void *)D.lists, (void *)D.list_row, (void *)D.list_slot})
+                if (p) cudaFree(p);
+        delete S;
+        S = nullptr;
+    }
+}
+
 static void free_layout(tfs_handle *h)
 {
     for (auto &kv : h->graphs) {
@@ -446,6 +478,7 @@ static void free_layout(tfs_handle *h)
                     h->d_lvl_begin, h->vec_pool, h->vec32_pool, h->part};
     for (void *p : ptrs)
         if (p) cudaFree(p);
+    free_tiles(h);
     h->perm = h->iperm = h->slice_off = h->col = h->vmap = nullptr;
     h->rowinfo = nullptr;
     h->val = nullptr;
@@ -546,6 +579,7 @@ static int build_layout(tfs_handle *h, int kind)
             vmap[(size_t)base + 32 * (size_t)j] = row0[o] + j;
         }
     }
+    h->perm_host = perm;
     h->n_int = n_int;
     h->n_chunks = n_int / TFS_TPB;
     h->n_slices = n_slices;
@@ -782,6 +816,7 @@ static int *option_field(tfs_handle *h, int option, bool (**ok)(int))
     case TFS_OPT_BWD_PRE: return &h->bwd_pre;
     case TFS_OPT_DIC_BLOCK: return &h->dic_block;
     case TFS_OPT_L2_WINDOW: return &h->l2_window;
+    case TFS_OPT_DIC_TILES: return &h->dic_tiles;
     default: return nullptr;
     }
 }
@@ -877,6 +912,125 @@ static cudaError_t launch_dic_one_block(tfs_handle *h, cudaStream_t s, int bytes
     return cudaPeekAtLastError();
 }
 
+// Whether the level kernels' own options are all at their defaults: one set
+// to another value selects the schedule that it shapes.
+static bool level_options_default(const tfs_handle *h)
+{
+    return h->tail_pf == 1 && h->fwd_pre == 1 && h->bwd_pre == 1;
+}
+
+// Most rows a plan may sweep per row: beyond it the tiles' closures outweigh
+// what the level launches cost.
+#define TFS_TILE_MAX_RATIO 2.2
+
+// Shared memory of a block's ring at most: what is in flight covers the
+// memory's latency well before this.
+#ifndef TFS_TILE_RING
+#define TFS_TILE_RING (96 << 10)
+#endif
+
+// The tiled DIC's plan for the current layout and arithmetic T, made on the
+// first DIC solve (the topology is fixed, so once per mesh).  A plan that does
+// not exist, or does not fit the room a server left, leaves tiles = 0: the
+// level kernels sweep.
+template <typename T>
+static int ensure_tiles(tfs_handle *h)
+{
+    TileStore *&S = h->tiles[sizeof(T) == 8];
+    if (!h->dic_tiles || h->layout != TFS_LAYOUT_LEVELS || !level_options_default(h) || S) return TFS_OK;
+    S = new TileStore;
+    int optin = 0;
+    CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
+    const int threads = std::max(1, std::min(16, (int)std::thread::hardware_concurrency()));
+    std::vector<int> internal(h->n);
+    for (int k = 0; k < h->n_int; k++)
+        if (h->perm_host[k] >= 0) internal[h->perm_host[k]] = k;
+    TilePlan P;
+    for (int tries = 0, tiles = tile_count(h->n, h->sm_count); tries < 2 && !P.tiles; tries++, tiles += h->sm_count)
+        P = tile_plan(h->n, h->row0, h->col0, h->dia0, h->levels_nat, h->rcm_pos, internal, tiles, TFS_TILE_MAX_RATIO,
+                      sizeof(T), optin, TFS_TILE_RING, threads);
+    if (!P.tiles) return TFS_OK;
+    int64_t bytes = 0;
+    for (TileDir &D : P.dir)
+        bytes += (int64_t)(D.rows.size() * 8 + D.packed.size() + D.rounds.size() * sizeof(TileRound) +
+                           D.list_row.size() * 6 + D.lists.size());
+    if (bytes > h->tile_room) return TFS_OK;
+    cudaStream_t s = h->stream;
+    int rc;
+    for (int d = 0; d < 2; d++) {
+        TileDir &D = P.dir[d];
+        TileStore::Dir &E = S->dir[d];
+        E.n_rounds = (int)D.rounds.size();
+        auto up = [&](auto **dst, const auto &src) -> int {
+            if (int rc = dalloc(h, dst, src.size())) return rc;
+            CK(cudaMemcpyAsync(*dst, src.data(), sizeof(src[0]) * src.size(), cudaMemcpyHostToDevice, s));
+            return TFS_OK;
+        };
+        if ((rc = up(&E.rounds, D.rounds)) || (rc = up(&E.tile_round, D.tile_round)) || (rc = up(&E.vbeg, D.vbeg)) ||
+            (rc = up(&E.rows, D.rows)) || (rc = up(&E.packed, D.packed)) || (rc = up(&E.tile_list, D.tile_list)) ||
+            (rc = up(&E.lists, D.lists)) || (rc = up(&E.list_row, D.list_row)) || (rc = up(&E.list_slot, D.list_slot))) {
+            cudaStreamSynchronize(s);
+            return rc;
+        }
+    }
+    CK(cudaStreamSynchronize(s));
+    CK(cudaFuncSetAttribute(k_dic_tile<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+    CK(cudaFuncSetAttribute(k_dic_tile<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+    S->max_slots = P.max_slots;
+    S->max_rounds = P.max_rounds;
+    S->max_lists = P.max_lists;
+    S->ring_bytes = P.ring_bytes;
+    S->smem_bytes = P.smem_bytes;
+    S->tiles = P.tiles;
+    h->stats.device_bytes = h->device_bytes;
+    return TFS_OK;
+}
+
+// Whether the sweeps of arithmetic T run tile by tile: a plan exists, and the
+// schedule is not one of the deep narrow ones that fit the one-block DIC.
+template <typename T>
+static bool use_tiles(const tfs_handle *h)
+{
+    const TileStore *S = h->tiles[sizeof(T) == 8];
+    return h->dic_tiles && S && S->tiles > 0 && !h->profiling && level_options_default(h) &&
+           !(h->n_levels >= TFS_DICB_SPLIT32_LEVELS && dic_block_kind<T>(h));
+}
+
+template <typename T>
+static TileDev tile_dev(const tfs_handle *h, int d)
+{
+    const TileStore &S = *h->tiles[sizeof(T) == 8];
+    const TileStore::Dir &E = S.dir[d];
+    return TileDev{E.rounds, E.tile_round, E.rows, E.vbeg, E.packed, E.tile_list, E.lists, E.list_row, E.list_slot,
+                   S.max_slots, S.max_rounds, S.max_lists, S.ring_bytes};
+}
+
+// D and the values of both directions into sweep order, after the factor is
+// formed; the number of kernels launched.
+template <typename T>
+static int launch_tile_fill(tfs_handle *h, cudaStream_t s)
+{
+    if (!use_tiles<T>(h)) return 0;
+    const TileStore &S = *h->tiles[sizeof(T) == 8];
+    k_tile_fill<T, 0><<<S.dir[0].n_rounds, TILE_ROWS, 0, s>>>(tile_dev<T>(h, 0), h->params, h->v.d);
+    k_tile_fill<T, 1><<<S.dir[1].n_rounds, TILE_ROWS, 0, s>>>(tile_dev<T>(h, 1), h->params, h->v.d);
+    return 2;
+}
+
+// z1 = M^-1 b1 tile by tile (y1: the start values between the sweeps).
+template <typename T>
+static int launch_tile_sweeps(tfs_handle *h, cudaStream_t s, const T *b1, T *y1, T *z1, int *count)
+{
+    const bool pdl = h->use_pdl != 0;
+    const TileStore &S = *h->tiles[sizeof(T) == 8];
+    cudaError_t e = launch_ex_smem(pdl, k_dic_tile<T, 0>, S.tiles, TILE_TPB, S.smem_bytes, s, tile_dev<T>(h, 0), b1, y1, h->st);
+    if (e == cudaSuccess)
+        e = launch_ex_smem(pdl, k_dic_tile<T, 1>, S.tiles, TILE_TPB, S.smem_bytes, s, tile_dev<T>(h, 1), (const T *)y1, z1, h->st);
+    *count += 2;
+    h->tiles_used = S.tiles;
+    return e == cudaSuccess ? TFS_OK : tfs_engine_error(e, "tiled DIC launch");
+}
+
 // DIC recurrence (Prec_Form.f90:32-40): one launch per large level, the tail
 // in one block, or the one-block kernel.  Returns the number of kernels
 // launched.
@@ -895,6 +1049,7 @@ static int launch_dic_form(tfs_handle *h, cudaStream_t s)
 
 static int tfs_mixed_prologue(tfs_handle *h, cudaStream_t s, int method, int prec, cudaGraphConditionalHandle cond);
 static int dic_l0_rows(const tfs_handle *h, int method, int prec);
+static int swept_l0_rows(const tfs_handle *h, int method, int prec);
 static int tfs_mixed_body(tfs_handle *h, cudaStream_t s, int method, int prec, cudaGraphConditionalHandle cond, int *count);
 static void tfs_mixed_fill32(tfs_handle *h, const double *src, float *dst);
 static void tfs_mixed_spmv_only(tfs_handle *h, cudaStream_t s);
@@ -911,13 +1066,16 @@ static int launch_prologue(tfs_handle *h, cudaStream_t s, int method, int prec,
                                   h->precision == TFS_MIXED ? h->val32 : nullptr, h->nnz_pad);
     k_load<<<G, T, 0, s>>>(A, h->val, h->perm, h->params, h->v, h->st, h->part, prec);
     *count = 3;
-    if (prec == 2) *count += launch_dic_form(h, s);
+    if (prec == 2) {
+        *count += launch_dic_form(h, s);
+        *count += h->precision == TFS_MIXED ? launch_tile_fill<float>(h, s) : launch_tile_fill<double>(h, s);
+    }
     if (h->precision == TFS_MIXED) {
         tfs_mixed_prologue(h, s, method, prec, cond);
         *count += 2;
     } else {
         if (method == TFS_CG) k_residual<0><<<G, T, 0, s>>>(A, h->val, h->v, h->st, h->part, prec, cond,
-                                                            dic_l0_rows(h, method, prec));
+                                                            swept_l0_rows(h, method, prec));
         else if (method == TFS_BICG) k_residual<1><<<G, T, 0, s>>>(A, h->val, h->v, h->st, h->part, prec, cond);
         else k_residual<2><<<G, T, 0, s>>>(A, h->val, h->v, h->st, h->part, prec, cond);
         *count += 1;
@@ -949,6 +1107,17 @@ static int launch_sweeps(tfs_handle *h, cudaStream_t s, int nr, const T *b1, con
     T *d;
     if constexpr (sizeof(T) == 8) { val = (const T *)h->val; d = (T *)h->v.d; }
     else { val = (const T *)h->val32; d = (T *)h->f.d; }
+    h->tiles_used = 0;
+    if (nr == 1 && use_tiles<T>(h)) {
+        h->dicb_used = 0;
+        int rc = launch_tile_sweeps<T>(h, s, b1, y1, z1, count);
+        if (rc || !fuse_l0) return rc;
+        const int l0 = h->lvl_begin[1];
+        cudaError_t e = launch_ex(h->use_pdl != 0, k_rho_l0<T>, (l0 + T_ - 1) / T_, T_, s, b1, (const T *)z1, l0,
+                                  h->n_int, h->st, h->part);
+        (*count)++;
+        return e == cudaSuccess ? TFS_OK : tfs_engine_error(e, "rho launch");
+    }
     if (nr == 1 && !fuse_l0) {
         int bytes = 0;
         if (dic_block_kind<T>(h, &bytes)) {
@@ -1030,6 +1199,14 @@ static int dic_l0_rows(const tfs_handle *h, int method, int prec)
     return h->lvl_begin[1];
 }
 
+// Rows whose forward sweep the update and residual kernels write: those of
+// dic_l0_rows, unless the tiles sweep every level.
+static int swept_l0_rows(const tfs_handle *h, int method, int prec)
+{
+    const int l0 = dic_l0_rows(h, method, prec);
+    return l0 && (h->precision == TFS_MIXED ? use_tiles<float>(h) : use_tiles<double>(h)) ? 0 : l0;
+}
+
 // After the binary64 preconditioner is formed: d32 = (float) d, then the
 // binary64 initial residual (k_mx_true<INIT>).
 static int tfs_mixed_prologue(tfs_handle *h, cudaStream_t s, int method, int prec,
@@ -1039,7 +1216,7 @@ static int tfs_mixed_prologue(tfs_handle *h, cudaStream_t s, int method, int pre
     const int G = h->grid, T = TFS_TPB;
     k_mx_cast<<<G, T, 0, s>>>(h->n_int, h->v.d, h->f.d);
     if (method == TFS_CG) k_mx_true<0, true><<<G, T, 0, s>>>(A, h->val, h->v, h->f, h->st, h->part, prec, cond,
-                                                             dic_l0_rows(h, method, prec));
+                                                             swept_l0_rows(h, method, prec));
     else if (method == TFS_BICG) k_mx_true<1, true><<<G, T, 0, s>>>(A, h->val, h->v, h->f, h->st, h->part, prec, cond);
     else k_mx_true<2, true><<<G, T, 0, s>>>(A, h->val, h->v, h->f, h->st, h->part, prec, cond);
     CKL("mixed prologue");
@@ -1075,7 +1252,7 @@ static int tfs_mixed_body(tfs_handle *h, cudaStream_t s, int method, int prec,
             k_mx_true<0, false><<<G, T, 0, s>>>(A, h->val, V, F, h->st, h->part, prec, cond);
             *count += 5;
         } else if (prec == 2 && dic_l0_rows(h, method, prec) > 0) {
-            const int l0 = dic_l0_rows(h, method, prec);
+            const int l0 = swept_l0_rows(h, method, prec);
             // The vector kernels after the sweeps are PDL-chained as well
             // (each waits for its predecessor before it reads anything).
             const bool pv = h->use_pdl && h->pdl_vec;
@@ -1171,7 +1348,7 @@ static int launch_body(tfs_handle *h, cudaStream_t s, int method, int prec,
     *count = 0;
     if (method == TFS_CG) {
         if (prec == 2 && dic_l0_rows(h, method, prec) > 0) {
-            const int l0 = dic_l0_rows(h, method, prec);
+            const int l0 = swept_l0_rows(h, method, prec);
             const bool pv = h->use_pdl && h->pdl_vec;   // vector kernels PDL-chained
             if ((rc = launch_sweeps<double>(h, s, 1, V.r, nullptr, V.y, nullptr, V.z, nullptr, count, true))) return rc;
             launch_ex(pv, k_cg_p<true>, G, T, s, nc, V, (const DevState *)h->st);
@@ -1417,6 +1594,7 @@ int tfs_solve_launch(int method, tfs_handle *h, const double *val, double *x, do
     CK(cudaSetDevice(h->device));
     int rc = ensure_layout(h, prec);
     if (rc) return rc;
+    if (prec == 2 && (rc = h->precision == TFS_MIXED ? ensure_tiles<float>(h) : ensure_tiles<double>(h))) return rc;
     // The reference's BiCG starts its shadow residual as r1 and drives it
     // with A, not A^T (Bicg.f90:91-93, 107-108, 136-144, 171-175): the shadow
     // sequence equals the primary one bit for bit, rho = (z1, r2) = (r1, z1)
@@ -1621,11 +1799,21 @@ static int vec_out(tfs_handle *h, const double *src, double *host)
     return TFS_OK;
 }
 
-static int form_prec(tfs_handle *h, int prec)
+// The preconditioner of h->val, and for DIC the tiles' packed values in the
+// arithmetic that is going to sweep.
+static int form_prec(tfs_handle *h, int prec, int mode = TFS_FP64)
 {
+    if (prec == 2) {
+        int rc = mode == TFS_FP64 ? ensure_tiles<double>(h) : ensure_tiles<float>(h);
+        if (rc) return rc;
+    }
     SellDev A = sell_of(h);
     k_diag_form<<<(h->n_int + 255) / 256, 256, 0, h->stream>>>(A, h->val, h->v.d, prec == 1 ? 1 : 0);
-    if (prec == 2) launch_dic_form(h, h->stream);
+    if (prec == 2) {
+        launch_dic_form(h, h->stream);
+        if (mode == TFS_FP64) launch_tile_fill<double>(h, h->stream);
+        else launch_tile_fill<float>(h, h->stream);
+    }
     CKL("prec form");
     return TFS_OK;
 }
@@ -1685,6 +1873,7 @@ extern "C" int tfs_get_stats(const tfs_handle *h, tfs_stats *out)
     out->spmv_kernel = h->spmv_kind;
     out->sell_width = h->sell_width;
     out->dic_kernel = h->dicb_used;
+    out->dic_tiles = h->tiles_used;
     return TFS_OK;
 }
 
@@ -1735,7 +1924,7 @@ extern "C" int tfs_time_prec(tfs_handle *h, const double *val, int mode, int rep
     CK(cudaSetDevice(h->device));
     int rc = prepare_values(h, val, 2);
     if (rc) return rc;
-    if ((rc = form_prec(h, 2))) return rc;
+    if ((rc = form_prec(h, 2, mode))) return rc;
     SellDev A = sell_of(h);
     cudaStream_t s = h->stream;
     k_diag_form<<<(h->n_int + 255) / 256, 256, 0, s>>>(A, h->val, h->v.r, 0);
@@ -1774,7 +1963,10 @@ extern "C" int tfs_profile_prec(tfs_handle *h, const double *val, int mode, int 
         (mode != TFS_FP64 && mode != TFS_MIXED))
         return TFS_ERR_ARG;
     double ms = 0.0;
+    const int keep_tiles = h->dic_tiles;
+    h->dic_tiles = 0;                               // the level launches are what is stamped
     int rc = tfs_time_prec(h, val, mode, 3, &ms);   // factor formed, warm
+    h->dic_tiles = keep_tiles;
     if (rc) return rc;
     if (h->dicb_used) {
         tfs_set_error_text("tfs_profile_prec: the one-block DIC has no level launches to stamp");
@@ -1840,18 +2032,25 @@ extern "C" int tfs_autotune(tfs_handle *h, const double *val, int mode, int prec
     memset(out, 0, sizeof(*out));
     int rc;
     if (prec == 2) {
+        // (the level kernels' block size: timed with the level kernels)
         static const int cand[4] = {128, 256, 512, 1024};
-        const int keep = h->level_tpb;
+        const int keep = h->level_tpb, keep_tiles = h->dic_tiles;
+        h->dic_tiles = 0;
         int best = keep;
         double best_ms = 0.0;
         for (int k = 0; k < 4; k++) {
             h->level_tpb = cand[k];
             double ms = 0.0;
-            if ((rc = tfs_time_prec(h, val, mode, reps, &ms))) { h->level_tpb = keep; return rc; }
+            if ((rc = tfs_time_prec(h, val, mode, reps, &ms))) {
+                h->level_tpb = keep;
+                h->dic_tiles = keep_tiles;
+                return rc;
+            }
             out->prec_ms[k] = ms;
             if (k == 0 || ms < best_ms) { best_ms = ms; best = cand[k]; }
         }
         h->level_tpb = best;
+        h->dic_tiles = keep_tiles;
     } else if ((rc = ensure_layout(h, prec))) {
         return rc;
     }

@@ -102,6 +102,7 @@ struct Vec32 {
 };
 
 struct FaceMap;   // tfs_assemble.cu
+struct TileStore; // tfs_engine.cu: the tiled DIC's plan on the device
 
 struct GraphEntry {
     cudaGraphExec_t exec = nullptr;
@@ -138,6 +139,10 @@ struct tfs_handle {
     int eager = 0;                     // TFS_OPT_LAUNCH: 1 launch kernels from a host loop, no CUDA graph
     int bicg_literal = 0;              // TFS_OPT_BICG: 1 BiCG runs its shadow sequence explicitly
     int dic_block = 1;                 // TFS_OPT_DIC_BLOCK: 1 one-block DIC where the vector and two slots of the widest level fit
+    int dic_tiles = 1;                 // TFS_OPT_DIC_TILES: 1 tiled DIC sweeps where the numbering allows
+    TileStore *tiles[2] = {nullptr, nullptr};   // binary32, binary64 plan of the current layout (null: not made yet)
+    int64_t tile_room = INT64_MAX;     // device bytes the plan may take (a server's budget)
+    int tiles_used = 0;                // tiles of the last DIC application launched (0: none)
     unsigned long long dicb_diag_ns = 0;   // tfs_diag_dic_timeout
     int l2_window = 1;                 // TFS_OPT_L2_WINDOW: 1 the column indices persisting in L2
     int dicb_used = 0;                 // the last DIC application launched was the one-block kernel
@@ -159,6 +164,7 @@ struct tfs_handle {
     uint64_t fingerprint = 0;
     std::vector<int> row0, col0, dia0;  // the topology, 0-based (host copy)
     std::vector<int> rcm_pos;          // RCM position of every natural row
+    std::vector<int> perm_host;        // natural row of every internal row, -1 padding (host copy of perm)
     int layout = -1;                   // TFS_LAYOUT_* built, -1 none yet
     int layout_pref = TFS_LAYOUT_RCM;  // TFS_OPT_LAYOUT = 1 forces level order
     int64_t fixed_bytes = 0;           // device bytes independent of the layout

@@ -12,6 +12,7 @@
 // at a time (a handle is not re-entrant); requests of one system are served
 // in arrival order.  Results do not depend on what else is running: each
 // solve has its own handle state and fixed-order reductions.
+#include <algorithm>
 #include <chrono>
 #include <condition_variable>
 #include <cstring>
@@ -154,6 +155,7 @@ static bool try_start(tfs_server *S, Request *r)
         S->stats.registrations++;
     }
     tfs_set_precision(sy.h, r->mode);
+    sy.h->tile_room = std::max<int64_t>(0, S->budget - S->resident);   // what a DIC tile plan may take
     r->t_start = clk::now();
     int rc = tfs_solve_launch(r->method, sy.h, r->val, r->x, r->r1, r->prec, r->niter, r->tol, !r->host,
                               r->host ? nullptr : r->b, r->x0_zero);

@@ -18,7 +18,7 @@ TFS_SYNTH_POISSON, TFS_SYNTH_CONVDIFF = 0, 1
 # options of a handle (tfs_set_option)
 (TFS_OPT_LAUNCH, TFS_OPT_LAYOUT, TFS_OPT_BICG, TFS_OPT_SELL_UNIFORM, TFS_OPT_SPMV, TFS_OPT_SPMV_GRID,
  TFS_OPT_LEVEL_TPB, TFS_OPT_TAIL_PF, TFS_OPT_FUSE_L0, TFS_OPT_PDL, TFS_OPT_PDL_VEC, TFS_OPT_FWD_PRE,
- TFS_OPT_BWD_PRE, TFS_OPT_DIC_BLOCK, TFS_OPT_L2_WINDOW) = range(1, 16)
+ TFS_OPT_BWD_PRE, TFS_OPT_DIC_BLOCK, TFS_OPT_L2_WINDOW, TFS_OPT_DIC_TILES) = range(1, 17)
 
 _PKG = Path(__file__).resolve().parent
 # TFS_LIBRARY selects another build of the library (same ABI).
@@ -40,7 +40,7 @@ class tfs_stats(C.Structure):
                 ("solve_ms", dbl), ("spmv_ns_total", dbl), ("spmv_launches", i64),
                 ("sweep_ns_total", dbl), ("sweep_launches", i64), ("kernel_launches", i64),
                 ("device_bytes", i64), ("spmv_kernel", i32), ("sell_width", i32),
-                ("dic_kernel", i32), ("pad", i32)]
+                ("dic_kernel", i32), ("dic_tiles", i32)]
 
 
 class tfs_result(C.Structure):
