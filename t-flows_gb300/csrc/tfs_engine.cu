@@ -103,22 +103,31 @@ static SellDev sell_of(const tfs_handle *h)
     return A;
 }
 
-// Kernel launch with programmatic dependent launch allowed (PDL) when pdl.
+// Kernel launch with programmatic dependent launch allowed (PDL) when pdl,
+// and with all of the unified L1 asked for when l1.
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_ex(bool pdl, void (*kernel)(KArgs...), int grid, int block, cudaStream_t s,
-                             Args... args)
+static cudaError_t launch_ex_l1(bool l1, bool pdl, void (*kernel)(KArgs...), int grid, int block, cudaStream_t s,
+                                Args... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3((unsigned)block);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
+    attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[1].val.sharedMemCarveout = cudaSharedmemCarveoutMaxL1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = l1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, ((KArgs)args)...);
+}
+
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_ex(bool pdl, void (*kernel)(KArgs...), int grid, int block, cudaStream_t s, Args... args)
+{
+    return launch_ex_l1(false, pdl, kernel, grid, block, s, args...);
 }
 
 // launch_ex with dynamic shared memory.
@@ -223,11 +232,25 @@ static void spmv_kind_setup(tfs_handle *h)
                                                                                 : TFS_SPMV_DIRECT;
 }
 
+// Rows from which the SpMV after tiled sweeps asks for all of the L1 (see
+// launch_spmv_pipe).
+#define TFS_SPMV_L1_ROWS (1 << 20)
+
 template <typename VT, bool MIXED>
 static void launch_spmv_pipe(const tfs_handle *h, cudaStream_t s, const VT *val, const VT *p, VT *q, bool pdl)
 {
     const SellDev A = sell_of(h);
     const int G = h->grid_spmv;
+    // The SpMV gathers through L1, and the multiprocessors keep the split of
+    // the sweeps before it, nearly all shared memory when those are tiled: a
+    // large SpMV asks for all of the L1 (binary64 100.7 -> 69.0 us on the
+    // 128^3 system, binary32 34.3 -> 30.0).  A small one would wait longer for
+    // the multiprocessors to change over than it gains (64^3 DIC-CG iteration
+    // 52.8 us without, 56.3 with; 1,320 cells 40.6 and 41.5).
+    const bool l1 = h->tiles_used && h->n_int >= TFS_SPMV_L1_ROWS;
+    auto launch_ex = [l1](bool on, auto kernel, int grid, int block, cudaStream_t st, auto... args) {
+        return launch_ex_l1(l1, on, kernel, grid, block, st, args...);
+    };
     switch (h->sell_width) {
     case 1: launch_ex(pdl, k_spmv_pq_pipe<VT, MIXED, 1>, G, TFS_TPB, s, A, val, p, q, h->st, h->part); break;
     case 2: launch_ex(pdl, k_spmv_pq_pipe<VT, MIXED, 2>, G, TFS_TPB, s, A, val, p, q, h->st, h->part); break;
