@@ -92,3 +92,27 @@ def test_faces_register_rejects_mismatch(gpu):
         with pytest.raises(TfsError):
             sol.assemble(np.zeros(len(faces)), np.zeros(len(faces)), np.zeros(len(faces)),
                          np.zeros(len(faces)))
+
+
+def hub_mesh(n, hub):
+    """A chain of n cells whose first cell is also joined to every cell from
+    3 to hub: one row of many entries among short ones."""
+    pairs = [(c, c + 1) for c in range(1, n)] + [(k, 1) for k in range(3, hub + 1)]
+    faces = np.array(pairs + [(c, -c) for c in range(1, n + 1, 5)], np.int32)
+    return faces[np.random.default_rng(n + hub).permutation(len(faces))]
+
+
+@pytest.mark.parametrize("n,hub", [(1, 0), (7, 0), (31, 8), (32, 9), (33, 20), (300, 299), (1000, 8)])
+def test_assemble_row_lengths(n, hub, gpu):
+    """Rows of at most eight entries are updated in shared memory, longer
+    ones in place, slices of 32 cells at a time."""
+    faces = hub_mesh(n, hub)
+    row, col, dia, mir, pos = O.topology(n, faces)
+    nf = len(faces)
+    rng = np.random.default_rng(n)
+    a12, a21, d12, d21 = (rng.uniform(0.1, 2.0, nf) for _ in range(4))
+    cell, start = rng.uniform(0.0, 1.0, n), rng.uniform(-1.0, 1.0, len(col))
+    want = O.assemble_faces(n, faces.reshape(-1), pos.reshape(-1), dia, a12, a21, d12, d21, cell, start)
+    with Solver(Matrix_Type(n, row, col, dia, want.copy())) as sol:
+        sol.faces_register(faces, pos)
+        assert np.array_equal(sol.assemble(a12, a21, d12, d21, cell, start), want)
