@@ -87,17 +87,26 @@ k_residual_norm_noalloc(int n, const int32_t *__restrict__ row1, const int32_t *
         r1[i] = r;
         e2 = r * r;
     }
-    __shared__ double sm[kRows / 32];
+    // The block's sum: every thread's square through shared memory, one warp
+    // adds kRows / 32 of them a lane and then across its lanes.  (Shuffles in
+    // every warp first were a quarter of the kernel's binary64 instructions,
+    // on the pipe that bounds it: 109 us a call on the 128^3 matrix, the copy
+    // of r1 included, against 97.  Products taken entry by entry into shared
+    // memory, so that values and columns are read coalesced, were slower, 115:
+    // the partly filled warps of a row's chain come on top.)
+    __shared__ double sm[kRows];
     __shared__ unsigned int is_last;
-    for (int o = 16; o > 0; o >>= 1) e2 = e2 + __shfl_down_sync(0xffffffffu, e2, o);
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = e2;
+    sm[threadIdx.x] = e2;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double s = sm[0];
-        for (int w = 1; w < kRows / 32; w++) s = s + sm[w];
-        scr->part[blockIdx.x] = s;
-        __threadfence();
-        is_last = (atomicAdd(&scr->counter, 1u) == gridDim.x - 1) ? 1u : 0u;
+    if (threadIdx.x < 32) {
+        double t = sm[threadIdx.x];
+        for (int w = 1; w < kRows / 32; w++) t = t + sm[32 * w + threadIdx.x];
+        for (int o = 16; o > 0; o >>= 1) t = t + __shfl_down_sync(0xffffffffu, t, o);
+        if (threadIdx.x == 0) {
+            scr->part[blockIdx.x] = t;
+            __threadfence();
+            is_last = (atomicAdd(&scr->counter, 1u) == gridDim.x - 1) ? 1u : 0u;
+        }
     }
     __syncthreads();
     if (!is_last) return;
