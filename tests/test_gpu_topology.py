@@ -47,3 +47,17 @@ def test_topology_device_edge_cases(gpu):
         Matrix_Mod_Topology_Device(2, np.array([[1, 3]], np.int32))     # cell out of range
     with pytest.raises(TfsError):
         Matrix_Mod_Topology_Device(2, np.array([[2, 2]], np.int32))     # c1 == c2
+
+
+@pytest.mark.parametrize("n,hub", [(7, 0), (255, 8), (256, 9), (257, 30), (3000, 2500), (2049, 8)])
+def test_topology_device_row_lengths(n, hub, gpu):
+    """Rows of at most eight entries are sorted in registers, longer ones in
+    place, 256 rows a block: a chain whose first cell is also joined to every
+    cell from 3 to hub."""
+    pairs = [(c, c + 1) for c in range(1, n)] + [(k, 1) for k in range(3, hub + 1)]
+    faces = np.array(pairs + [(c, -c) for c in range(1, n + 1, 7)], np.int32)
+    faces = np.ascontiguousarray(faces[np.random.default_rng(n).permutation(len(faces))])
+    row, col, dia, mir, pos = O.topology(n, faces)
+    dev = Matrix_Mod_Topology_Device(n, faces)
+    assert np.array_equal(dev.row, row) and np.array_equal(dev.col, col)
+    assert np.array_equal(dev.dia, dia) and np.array_equal(dev.mir, mir) and np.array_equal(dev.pos, pos)
