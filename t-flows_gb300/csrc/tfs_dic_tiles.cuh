@@ -39,6 +39,7 @@ constexpr int TILE_TPB = TILE_ROWS + 2 * TILE_MOVERS + 32;   // row threads, loa
 #ifndef TFS_TILE_BATCH
 #define TFS_TILE_BATCH 8
 #endif
+constexpr int TILE_QUIT = 2;                              // abort flag of a sweep that has nothing to do
 constexpr int TILE_BATCH = TFS_TILE_BATCH;                // list rounds whose rows a mover holds at once
 
 // One direction of a plan on the device.
@@ -172,7 +173,7 @@ __device__ __forceinline__ void tile_move(const TileDev &P, int m, const T *src,
     cudaGridDependencySynchronize();
     const unsigned long long diag = st->dicb_wait_ns;
     const unsigned long long wait_ns = diag ? diag : TFS_DICB_WAIT_NS;
-    const bool skip = st->done != 0;
+    if (st->done) return;
     for (int q0 = 0; q0 < n; q0 += TILE_BATCH) {
 #pragma unroll
         for (int u = 0; u < TILE_BATCH; u++) {
@@ -180,7 +181,7 @@ __device__ __forceinline__ void tile_move(const TileDev &P, int m, const T *src,
             const uint8_t l = lists[q0 + u];
             if (STORE) {
                 tile_wait(done + (l & 127u), 0u, abort, wait_ns);
-                if ((w[u] & TILE_OWN) && !skip) dst[w[u] & TILE_ROW_MASK] = s[k[u]];
+                if (w[u] & TILE_OWN) dst[w[u] & TILE_ROW_MASK] = s[k[u]];
             } else {
                 if ((w[u] & TILE_ROW_MASK) != TILE_NO_ROW)
                     tile_cp_async(s_at + k[u] * (uint32_t)sizeof(T), src + (w[u] & TILE_ROW_MASK));
@@ -275,7 +276,10 @@ k_dic_tile(TileDev P, const T *__restrict__ src, T *__restrict__ dst, DevState *
     cudaGridDependencySynchronize();
     const unsigned long long diag = st->dicb_wait_ns;
     const unsigned long long wait_ns = diag ? diag : TFS_DICB_WAIT_NS;
-    const bool skip = st->done != 0;
+    if (st->done) {          // nothing to sweep: the copy lane leaves as after an abort
+        if (tid == 0) *abort = TILE_QUIT;
+        return;
+    }
     if (DIR == 0 && blockIdx.x == 0 && tid == 0) st->t_sweep0 = gtimer();
     int level = 0;
     bool ok = tile_wait(loaded, 0u, abort, wait_ns);
@@ -320,7 +324,7 @@ k_dic_tile(TileDev P, const T *__restrict__ src, T *__restrict__ dst, DevState *
             if (MOVED && tid == 0) dicb_mbar_arrive(done + level);
             level++;
         }
-        if (!MOVED && (w & TILE_OWN) && !skip) dst[w & TILE_ROW_MASK] = DIR == 0 ? tile_quotient(acc, y, d, rc) : y;
+        if (!MOVED && (w & TILE_OWN)) dst[w & TILE_ROW_MASK] = DIR == 0 ? tile_quotient(acc, y, d, rc) : y;
     }
     tile_row_sync();
     if (tid == 0 && *abort) {
