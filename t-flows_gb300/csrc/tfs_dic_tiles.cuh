@@ -140,6 +140,24 @@ __device__ __noinline__ bool tile_wait_slow(uint64_t *bar, unsigned parity, vola
 {
     return dicb_mbar_wait(bar, parity, abort, wait_ns);
 }
+// The copy lane's wait for a release: it looks at the abort flag between two
+// tests that do not suspend it (try_wait may for a good part of a
+// millisecond, which a sweep with nothing to do would spend leaving).
+__device__ __forceinline__ bool tile_wait_empty(uint64_t *bar, unsigned parity, volatile int *abort, unsigned long long wait_ns)
+{
+    const unsigned long long t0 = gtimer();
+    for (;;) {
+        unsigned ok;
+        asm volatile("{ .reg .pred p; mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                     : "=r"(ok) : "r"(dicb_smem_addr(bar)), "r"(parity) : "memory");
+        if (ok) return true;
+        if (*abort) return false;
+        if (gtimer() - t0 > wait_ns) {
+            *abort = 1;
+            return false;
+        }
+    }
+}
 __device__ __forceinline__ bool tile_wait(uint64_t *bar, unsigned parity, volatile int *abort, unsigned long long wait_ns)
 {
     return dicb_mbar_test(bar, parity) || tile_wait_slow(bar, parity, abort, wait_ns);
@@ -257,7 +275,7 @@ k_dic_tile(TileDev P, const T *__restrict__ src, T *__restrict__ dst, DevState *
         for (; k < rounds && !*abort; k++) {
             const uint4 c = tab[k];
             const int back = (int)(c.y >> 16 & 0xffu), dep = k - back;
-            if (back && !dicb_mbar_wait(empty + dep % TILE_BARS, (unsigned)(dep / TILE_BARS) & 1u, abort, wait_ns)) break;
+            if (back && !tile_wait_empty(empty + dep % TILE_BARS, (unsigned)(dep / TILE_BARS) & 1u, abort, wait_ns)) break;
             uint64_t *bar = full + k % TILE_BARS;
             const unsigned bytes = (c.y & 0xffffu) * 16u;
             dicb_mbar_expect(bar, bytes);
@@ -276,7 +294,7 @@ k_dic_tile(TileDev P, const T *__restrict__ src, T *__restrict__ dst, DevState *
     cudaGridDependencySynchronize();
     const unsigned long long diag = st->dicb_wait_ns;
     const unsigned long long wait_ns = diag ? diag : TFS_DICB_WAIT_NS;
-    if (st->done) {          // nothing to sweep: the copy lane leaves as after an abort
+    if (st->done) {   // nothing to sweep: the copy lane leaves as after an abort
         if (tid == 0) *abort = TILE_QUIT;
         return;
     }
@@ -367,7 +385,7 @@ k_rho_l0(const T *__restrict__ r, const T *__restrict__ z, int l0_rows, int n_in
 {
     cudaGridDependencySynchronize();
     cudaTriggerProgrammaticLaunchCompletion();
-    const bool stop = (st->done | st->need_true) != 0;
+    const bool stop = (st->done) != 0;
     const int i = blockIdx.x * TFS_TPB + threadIdx.x;
     T acc = (T)0;
     if (i < l0_rows) {
