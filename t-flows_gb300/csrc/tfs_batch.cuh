@@ -53,84 +53,106 @@ struct BatchSys {
     double ini_res, fin_res;
 };
 
+static_assert(sizeof(BatchSys) % 8 == 0, "copied to shared memory by words of eight bytes");
+
 struct BatchCtl {
     unsigned int head;        // next queue position
     unsigned int pad;
 };
 
 #define TFS_BATCH_MAX_TPB 512
-// Resident CTAs of 512 threads per SM the kernel is compiled for (at most
-// 65536 / (512 * 3) = 42 registers, with some spilling).  Measured on the
-// 256-system batch (mixed, best cluster shape each): 1 -> 422, 2 -> 499,
-// 3 -> 584, 4 -> 545 solves/s; the latency-bound solves gain more from
-// resident warps than they lose to the spills.
-#ifndef TFS_BATCH_MIN_BLOCKS
-#define TFS_BATCH_MIN_BLOCKS 3
-#endif
+// CTAs of 512 threads an SM is to hold: one (128 registers, no spilling) or,
+// for binary32 batches that ask for more CTAs than TFS_BATCH_ROOMY an SM, two
+// (64 registers, 90 bytes spilled).  Measured, one / two, ms: 24 systems of
+// 5k to 91k cells mixed 16 x 512 10.6 / 10.2, 8 x 512 9.6 / 14.0; 96 systems
+// of up to 500k cells mixed 16 x 512 235 / 197, 8 x 512 221 / 215; binary64
+// 24 systems 27.7 / 31.7 and 39.9 / 43.6, 96 systems 608 / 583 and 539 / 569.
+// (Three, as long as the whole system's pointers and every thread's copy of
+// the solve's scalars were spilled: 20.8 and 21.5, 249 and 353; binary64 45.8
+// and 48.7, 622 and 751.)
+#define TFS_BATCH_ROOMY 3
 
 // Sum of NV values over the cluster: block sum, one partial per CTA in
-// shared memory, cluster barrier, every thread adds the C partials in rank
-// order.  Two partial slots alternate, so a slot is rewritten only after the
-// next barrier, by which time every reader of its previous contents is done.
+// shared memory, cluster barrier, the C partials added in rank order.  The
+// totals are valid in thread 0 of every CTA (all get the same bits), which
+// alone goes on with them: a binary64 instruction occupies a quarter of an
+// SM's narrow binary64 pipe for 64 cycles a warp, and when every thread
+// added the partials and took the divisions and square roots of an iteration
+// itself, those hundred instructions in 16 warps were most of a small
+// system's iteration.  Two partial slots alternate, so a slot is rewritten
+// only after the next barrier, by which time every reader of its previous
+// contents is done.
 //
 // AT is the type of the per-thread partials: binary64, or binary32 in the
-// mixed solves, whose warp sums then go through warp_sum_f (compensated
-// binary32, no binary64 instruction per lane).
+// mixed solves, whose warp sums are compensated pairs (warp_sum_f2), turned
+// into binary64 a lane per warp by the first warp.
 template <int NV, typename AT = double>
 __device__ __forceinline__ void cluster_sum(const AT (&in)[NV], double (&v)[NV], double (*s_part)[4],
                                             int &parity, cg::cluster_group &cl)
 {
     __shared__ double sm[NV][TFS_BATCH_MAX_TPB / 32];
+    __shared__ float smf[NV][2][TFS_BATCH_MAX_TPB / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
     for (int k = 0; k < NV; k++) {
-        double w;
         if constexpr (sizeof(AT) == 4) {
-            w = warp_sum_f(in[k]);
+            float hi, lo;
+            warp_sum_f2(in[k], hi, lo);
+            if (lane == 0) { smf[k][0][warp] = hi; smf[k][1][warp] = lo; }
         } else {
-            w = in[k];
+            double w = in[k];
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) w = w + __shfl_down_sync(FULL, w, o);
+            if (lane == 0) sm[k][warp] = w;
         }
-        if (lane == 0) sm[k][warp] = w;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (warp == 0) {
+        if constexpr (sizeof(AT) == 4) {
 #pragma unroll
-        for (int k = 0; k < NV; k++) {
-            double s = sm[k][0];
-            for (int w = 1; w < nw; w++) s = s + sm[k][w];
-            s_part[parity][k] = s;
+            for (int k = 0; k < NV; k++)
+                if (lane < nw) sm[k][lane] = (double)smf[k][0][lane] + (double)smf[k][1][lane];
+            __syncwarp();
+        }
+        if (lane < NV) {   // one value a lane
+            double s = sm[lane][0];
+            for (int w = 1; w < nw; w++) s = s + sm[lane][w];
+            s_part[parity][lane] = s;
         }
     }
     cl.sync();
-    const unsigned C = cl.num_blocks();
-#pragma unroll
-    for (int k = 0; k < NV; k++) {
+    if (warp == 0) {
+        const unsigned C = cl.num_blocks();
         double s = 0.0;
-        for (unsigned r = 0; r < C; r++) {
-            double(*rp)[4] = cl.map_shared_rank(s_part, r);
-            s = s + rp[parity][k];
+        if (lane < NV) {
+#pragma unroll 8
+            for (unsigned r = 0; r < C; r++) {
+                double(*rp)[4] = cl.map_shared_rank(s_part, r);
+                s = s + rp[parity][lane];
+            }
         }
-        v[k] = s;
+#pragma unroll
+        for (int k = 0; k < NV; k++) v[k] = __shfl_sync(FULL, s, k);
     }
     parity ^= 1;
 }
 
+// The vectors of arithmetic VT, by name.  S lies in shared memory and each
+// phase of a solve takes the few pointers that it uses: thirty-odd pointers
+// kept in registers through the whole solve were spilled, and with them the
+// solve's own values.
 template <typename VT>
-struct BatchVecs;
-template <>
-struct BatchVecs<double> {
-    double *r, *r2, *p, *p2, *q, *q2, *z, *z2;
-    __device__ BatchVecs(const BatchSys &S)
-        : r(S.V.r), r2(S.V.r2), p(S.V.p), p2(S.V.p2), q(S.V.q), q2(S.V.q2), z(S.V.z), z2(S.V.z2) {}
-};
-template <>
-struct BatchVecs<float> {
-    float *r, *r2, *p, *p2, *q, *q2, *z, *z2;
-    __device__ BatchVecs(const BatchSys &S)
-        : r(S.F.r), r2(S.F.r2), p(S.F.p), p2(S.F.p2), q(S.F.q), q2(S.F.q2), z(S.F.z), z2(S.F.z2) {}
-};
+__device__ __forceinline__ auto &batch_vecs(BatchSys &S)
+{
+    if constexpr (sizeof(VT) == 4) return S.F;
+    else return S.V;
+}
+template <typename VT>
+__device__ __forceinline__ const VT *batch_val(const BatchSys &S)
+{
+    if constexpr (sizeof(VT) == 4) return S.val32;
+    else return S.val;
+}
 
 // The whole solve of one system by the calling cluster.  VT = double:
 // binary64 with the reference's per-row arithmetic; VT = float: mixed.
@@ -211,265 +233,368 @@ __device__ AccT batch_dic_apply(const SellDev &A, const VT *val, const VT *d, co
     return rz;
 }
 
+// q = A p over the thread's rows (gtid, gtid + stride, ...) and its partial
+// of (p, q).  Uniform slice widths up to 8 (hex meshes) run software-pipelined
+// as k_spmv_pq_pipe does: the next row's columns are loaded while the gathers
+// and values of the current one are in flight.  Gathers past L1: other CTAs
+// of the cluster wrote p.
+template <typename VT, typename AccT>
+__device__ __forceinline__ void batch_spmv(const SellDev &A, const VT *__restrict__ val, const VT *p, VT *q, AccT &pq,
+                                           int n_int, int gtid, int stride)
+{
+    if (A.width > 0 && A.width <= 8) {
+        constexpr int W = 8;
+        int nk[W];
+        uint32_t ninfo = 0u;
+        auto cols = [&](int i) {
+            const int off = (i & ~31) * A.width + (i & 31);
+            ninfo = __ldg(A.rowinfo + i);
+#pragma unroll
+            for (int j = 0; j < W; j++)
+                if (j < A.width) nk[j] = __ldg(A.col + off + 32 * j);
+        };
+        if (gtid < n_int) cols(gtid);
+        for (int i = gtid; i < n_int; i += stride) {
+            const int off = (i & ~31) * A.width + (i & 31), len = (int)(ninfo & 0xffffu);
+            VT x[W], a[W];
+#pragma unroll
+            for (int j = 0; j < W; j++)
+                if (j < len) {
+                    x[j] = __ldcg(p + nk[j]);
+                    a[j] = __ldg(val + off + 32 * j);
+                }
+            const VT pi = p[i];
+            if (i + stride < n_int) cols(i + stride);
+            VT s = (VT)0;
+#pragma unroll
+            for (int j = 0; j < W; j++)
+                if (j < len) s = s + a[j] * x[j];
+            q[i] = s;
+            pq = acc_fma(pi, s, pq);
+        }
+        return;
+    }
+    for (int i = gtid; i < n_int; i += stride) {
+        const RowGeom g = row_geom(A, i);
+        const VT s = row_accum<false, VT, VT, VT, false, 4>((VT)0, A.col, val, p, g.off, 0, g.len);
+        q[i] = s;
+        pq = acc_fma(p[i], s, pq);
+    }
+}
+
+// What thread 0 of a CTA keeps and hands to the others, in shared memory.
+struct BatchLead {
+    double alfa, beta;                            // for every thread
+    int need, done;                               // (two words: each is read while thread 0 may already write the other)
+    double err, ini, rho, rho_old, r_true;        // thread 0's own
+    int status, niter_out, early, true_res;
+};
+
+// r = b - A x in binary64 (b in V.u1), the iteration's residual and, unless
+// DIC sweeps do it, z = M^-1 r; the thread's partials of ||r||^2 and rho.
 template <int METHOD, typename VT>
-__device__ void batch_solve_one(BatchSys &S, cg::cluster_group &cl, double (*s_part)[4], int &parity)
+__device__ __forceinline__ void batch_true_residual(BatchSys &S, int gtid, int stride, double &e2, double &rz)
+{
+    constexpr bool MIXED = sizeof(VT) == 4;
+    const SellDev A = S.A;
+    const double *const val = S.val, *const b = S.V.u1, *const x = S.V.x;
+    double *const r64 = S.V.r;
+    auto &W = batch_vecs<VT>(S);
+    VT *const rT = W.r, *const z = W.z, *const r2 = W.r2, *const z2 = W.z2;
+    const VT *const d = W.d;
+    e2 = 0.0;
+    rz = 0.0;
+    for (int i = gtid; i < A.n_int; i += stride) {
+        const RowGeom g = row_geom(A, i);
+        const double r = row_accum<true, double, double, double, false, 4>(b[i], A.col, val, x, g.off, 0, g.len);
+        r64[i] = r;
+        e2 = fma(r, r, e2);
+        const VT rt = (VT)r;
+        if (MIXED) rT[i] = rt;
+        if (METHOD == 2) continue;   // z and (r, z) from the sweeps
+        const VT zt = rt / d[i];
+        z[i] = zt;
+        if (METHOD == 1) {
+            // The shadow residual equals r1 (see k_mx_true): reset both.
+            r2[i] = rt;
+            z2[i] = zt;
+            rz = fma((double)zt, (double)rt, rz);
+        } else {
+            rz = fma((double)rt, (double)zt, rz);
+        }
+    }
+}
+
+// z = M^-1 r by the DIC sweeps; the thread's partial of (r, z).
+template <typename VT, typename AccT>
+__device__ __forceinline__ AccT batch_sweeps(BatchSys &S, int gtid, int stride, cg::cluster_group &cl)
+{
+    cl.sync();
+    const SellDev A = S.A;
+    auto &W = batch_vecs<VT>(S);
+    return batch_dic_apply<VT, AccT>(A, batch_val<VT>(S), (const VT *)W.d, W.r, W.y, W.z, S.lvl_begin, S.n_levels,
+                                     gtid, stride, cl);
+}
+
+template <int METHOD, typename VT>
+__device__ void batch_solve_one(BatchSys &S, BatchSys &out, BatchLead &L, cg::cluster_group &cl, double (*s_part)[4],
+                                int &parity)
 {
     constexpr bool MIXED = sizeof(VT) == 4;
     using AccT = VT;
-    const int C = (int)cl.num_blocks();
-    const int stride = C * (int)blockDim.x;
+    const int stride = (int)cl.num_blocks() * (int)blockDim.x;
     const int gtid = (int)cl.block_rank() * (int)blockDim.x + (int)threadIdx.x;
-    const SellDev A = S.A;
-    const int n_int = A.n_int;
-    const Vec64 V = S.V;
-    const Vec32 F = S.F;
-    BatchVecs<VT> W(S);
-    const VT *valT;
-    if constexpr (MIXED) valT = S.val32; else valT = S.val;
-    const double tol = S.tol;
-    const int niter_max = S.niter_max;
-    const bool diag = S.prec == 1;
+    const int n_int = S.A.n_int;
     // METHOD 2: the CG sequence with DIC preconditioning (its own instance,
     // so that the DIC sweeps add no registers to the other kernels)
     constexpr bool dic = METHOD == 2;
-    VT *yT;
-    if constexpr (MIXED) yT = F.y; else yT = V.y;
+    const bool lead = threadIdx.x == 0;
+    auto &W = batch_vecs<VT>(S);
 
     // b, x0 in internal order, d, ||b|| (Cg.f90:48-58).  The values were
     // gathered into SELL order by k_batch_gather before this launch.
-    double acc[2] = {0.0, 0.0};
-    for (int i = gtid; i < n_int; i += stride) {
-        int o = __ldg(S.perm + i);
-        double bi = 0.0, xi = 0.0;
-        if (o >= 0) { bi = S.b[o]; xi = S.x[o]; }
-        V.r[i] = bi;
-        V.u1[i] = bi;
-        V.x[i] = xi;
-        acc[0] = fma(bi, bi, acc[0]);
-    }
-    for (int i = gtid; i < n_int; i += stride) {
-        RowGeom g = row_geom(A, i);
-        double di = (diag && g.len > 0) ? S.val[g.off + (g.dpos << 5)] : 1.0;
-        V.d[i] = di;
-        if (MIXED) { F.d[i] = (float)di; F.e[i] = 0.f; }
-    }
-    if (dic) {
-        cl.sync();
-        batch_dic_form(A, S.val, V.d, S.lvl_begin, S.n_levels, gtid, stride, cl);
-        if (MIXED)
-            for (int i = gtid; i < n_int; i += stride) F.d[i] = (float)__ldcg(V.d + i);
-    }
     {
-        const double a1[1] = {acc[0]};
-        double v1[1];
-        cluster_sum<1>(a1, v1, s_part, parity, cl);
-        double bnrm2 = sqrt(v1[0]);
-        if (bnrm2 < tol) {
-            // Early exit 1: x, r1 untouched, ini_res untouched (Cg.f90:55-58).
-            if (cl.block_rank() == 0 && threadIdx.x == 0) {
-                S.niter_out = 0; S.early = 1; S.fin_res = bnrm2; S.status = TFS_OK; S.true_res = 0;
-            }
-            return;
-        }
-    }
-    // True residual r = b - A x; r2 = r (shadow); z = M^-1 r; ||r0||; rho.
-    auto true_residual = [&](bool init, double &e2, double &rz) {
-        e2 = 0.0;
-        rz = 0.0;
-        for (int i = gtid; i < n_int; i += stride) {
-            RowGeom g = row_geom(A, i);
-            double r = row_accum<true, double, double, double, false, 4>(V.u1[i], A.col, S.val, V.x, g.off, 0, g.len);
-            V.r[i] = r;
-            e2 = fma(r, r, e2);
-            VT rT = (VT)r;
-            if (MIXED) W.r[i] = rT;
-            if (dic) continue;   // z and (r, z) from the sweeps below
-            VT dT = MIXED ? (VT)F.d[i] : (VT)V.d[i];
-            VT z = rT / dT;
-            W.z[i] = z;
-            if (METHOD == 1) {
-                // The shadow residual equals r1 (see k_mx_true): reset both.
-                W.r2[i] = rT;
-                W.z2[i] = z;
-                rz = fma((double)z, (double)rT, rz);
-            } else {
-                rz = fma((double)rT, (double)z, rz);
-            }
-        }
-    };
-    double e2, rz;
-    true_residual(true, e2, rz);
-    if (dic) {
-        cl.sync();
-        rz = (double)batch_dic_apply<VT, double>(A, valT, MIXED ? (const VT *)F.d : (const VT *)V.d, W.r, yT, W.z,
-                                                 S.lvl_begin, S.n_levels, gtid, stride, cl);
-    }
-    const double a2[2] = {e2, rz};
-    double v2[2];
-    cluster_sum<2>(a2, v2, s_part, parity, cl);
-    double err = sqrt(v2[0]);
-    double ini = err, rho = v2[1], rho_old = 0.0, r_true = err;
-    int true_res = 1, status = TFS_OK, niter_out = 0, early = 0;
-    int iter = 1;
-    bool done = false;
-    if (!(err <= DBL_MAX)) { status = TFS_ERR_NONFINITE; niter_out = (niter_max > 0 ? niter_max : 0) + 1; done = true; }
-    else if (err < tol) { niter_out = 0; early = 2; done = true; }
-    else if (niter_max <= 0) { niter_out = 1; done = true; }
-
-    while (!done) {
-        // p = z + beta p (Cg.f90:114-123; both directions for BiCG).
-        const double beta = iter == 1 ? 0.0 : rho / rho_old;
-        const VT betaT = (VT)beta;
-        for (int i0 = gtid; i0 < n_int; i0 += 2 * stride) {
-            const int i1 = i0 + stride;
-            const bool ok1 = i1 < n_int;
-            // z past L1: with DIC other threads of the cluster wrote it
-            VT z0 = __ldcg(W.z + i0), p0 = W.p[i0], z1 = ok1 ? __ldcg(W.z + i1) : (VT)0,
-               p1 = ok1 ? W.p[i1] : (VT)0;
-            VT a0 = (VT)0, b0 = (VT)0, a1 = (VT)0, b1 = (VT)0;
-            if (METHOD == 1) {
-                a0 = W.z2[i0]; b0 = W.p2[i0];
-                if (ok1) { a1 = W.z2[i1]; b1 = W.p2[i1]; }
-            }
-            W.p[i0] = iter == 1 ? z0 : z0 + betaT * p0;
-            if (METHOD == 1) W.p2[i0] = iter == 1 ? a0 : a0 + betaT * b0;
-            if (ok1) {
-                W.p[i1] = iter == 1 ? z1 : z1 + betaT * p1;
-                if (METHOD == 1) W.p2[i1] = iter == 1 ? a1 : a1 + betaT * b1;
-            }
-        }
-        cl.sync();
-        // q = A p and alpha (Cg.f90:128-153 / Bicg.f90:136-165).
-        AccT pq = (AccT)0;
-        if (METHOD == 1) {
+        double acc = 0.0;
+        {
+            const int *const perm = S.perm;
+            const double *const b = S.b, *const x0 = S.x;
+            double *const r = S.V.r, *const u = S.V.u1, *const x = S.V.x;
             for (int i = gtid; i < n_int; i += stride) {
-                RowGeom g = row_geom(A, i);
-                VT s1 = (VT)0, s2 = (VT)0;
-                row_accum2<false, VT, VT, VT>(s1, s2, A.col, valT, W.p, W.p2, g.off, 0, g.len);
-                W.q[i] = s1;
-                W.q2[i] = s2;
-                pq = acc_fma(W.p2[i], s1, pq);
-            }
-        } else {
-            // Four rows per thread and step, all loads before any store.
-            for (int i0 = gtid; i0 < n_int; i0 += 4 * stride) {
-                int ii[4];
-                VT sv[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    ii[q] = i0 + q * stride;
-                    sv[q] = (VT)0;
-                    if (ii[q] < n_int) {
-                        RowGeom g = row_geom(A, ii[q]);
-                        sv[q] = row_accum<false, VT, VT, VT, false, 4>((VT)0, A.col, valT, W.p, g.off, 0, g.len);
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < 4; q++)
-                    if (ii[q] < n_int) {
-                        W.q[ii[q]] = sv[q];
-                        pq = acc_fma(W.p[ii[q]], sv[q], pq);
-                    }
+                const int o = __ldg(perm + i);
+                double bi = 0.0, xi = 0.0;
+                if (o >= 0) { bi = b[o]; xi = x0[o]; }
+                r[i] = bi;
+                u[i] = bi;
+                x[i] = xi;
+                acc = fma(bi, bi, acc);
             }
         }
-        const AccT a1[1] = {pq};
-        double v1[1];
-        cluster_sum<1, AccT>(a1, v1, s_part, parity, cl);
-        const double alfa = rho / v1[0];
-        const VT alfaT = (VT)alfa;
-        // x (or e) += alpha p, r -= alpha q, z = M^-1 r, ||r||, next rho.
-        AccT e2a = (AccT)0, rza = (AccT)0;
-        if (METHOD == 1) {
+        {
+            const SellDev A = S.A;
+            const double *const val = S.val;
+            const bool diag = S.prec == 1;
+            double *const d = S.V.d;
+            float *const d32 = S.F.d, *const e = S.F.e;
             for (int i = gtid; i < n_int; i += stride) {
-                if (MIXED) F.e[i] = fmaf((float)alfaT, (float)W.p[i], F.e[i]);
-                else V.x[i] = V.x[i] + alfa * (double)W.p[i];
-                VT r1 = W.r[i] - alfaT * W.q[i];
-                W.r[i] = r1;
-                VT dT = MIXED ? (VT)F.d[i] : (VT)V.d[i];
-                VT z1 = r1 / dT;
-                W.z[i] = z1;
-                e2a = acc_fma(r1, r1, e2a);
-                VT r2 = W.r2[i] - alfaT * W.q2[i];
-                W.r2[i] = r2;
-                W.z2[i] = r2 / dT;
-                rza = acc_fma(z1, r2, rza);
-            }
-        } else {
-            for (int i0 = gtid; i0 < n_int; i0 += 4 * stride) {
-                int ii[4];
-                VT pv[4], rv[4], qv[4], dv[4];
-                double xv[4];
-                float ev[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    ii[q] = i0 + q * stride;
-                    const int i = ii[q] < n_int ? ii[q] : i0;
-                    pv[q] = W.p[i]; rv[q] = W.r[i]; qv[q] = W.q[i];
-                    dv[q] = MIXED ? (VT)F.d[i] : (VT)V.d[i];
-                    if (MIXED) ev[q] = F.e[i]; else xv[q] = V.x[i];
-                }
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    if (ii[q] >= n_int) continue;
-                    const int i = ii[q];
-                    if (MIXED) F.e[i] = fmaf((float)alfaT, (float)pv[q], ev[q]);
-                    else V.x[i] = xv[q] + alfa * (double)pv[q];
-                    VT r1 = rv[q] - alfaT * qv[q];
-                    W.r[i] = r1;
-                    e2a = acc_fma(r1, r1, e2a);
-                    if (dic) continue;
-                    VT z1 = r1 / dv[q];
-                    W.z[i] = z1;
-                    rza = acc_fma(r1, z1, rza);
-                }
+                const RowGeom g = row_geom(A, i);
+                const double di = (diag && g.len > 0) ? val[g.off + (g.dpos << 5)] : 1.0;
+                d[i] = di;
+                if (MIXED) { d32[i] = (float)di; e[i] = 0.f; }
             }
         }
         if (dic) {
             cl.sync();
-            rza = batch_dic_apply<VT, AccT>(A, valT, MIXED ? (const VT *)F.d : (const VT *)V.d, W.r, yT, W.z,
-                                            S.lvl_begin, S.n_levels, gtid, stride, cl);
+            const SellDev A = S.A;
+            batch_dic_form(A, S.val, S.V.d, S.lvl_begin, S.n_levels, gtid, stride, cl);
+            if (MIXED) {
+                const double *const d = S.V.d;
+                float *const d32 = S.F.d;
+                for (int i = gtid; i < n_int; i += stride) d32[i] = (float)__ldcg(d + i);
+            }
         }
-        const AccT a3[2] = {e2a, rza};
-        double v3[2];
-        cluster_sum<2, AccT>(a3, v3, s_part, parity, cl);
-        double est = sqrt(v3[0]);
-        double rho_next = v3[1];
-        bool need_true = MIXED && (!(est <= DBL_MAX) || est < tol || est < 0.1 * r_true || iter >= niter_max);
-        if (need_true) {
-            for (int i = gtid; i < n_int; i += stride) {
-                V.x[i] = V.x[i] + (double)F.e[i];
-                F.e[i] = 0.f;
+        const double a1[1] = {acc};
+        double v1[1];
+        cluster_sum<1>(a1, v1, s_part, parity, cl);
+        if (lead) {
+            const double bnrm2 = sqrt(v1[0]);
+            L.done = bnrm2 < S.tol;
+            if (L.done && cl.block_rank() == 0) {
+                // Early exit 1: x, r1 untouched, ini_res untouched (Cg.f90:55-58).
+                out.niter_out = 0; out.early = 1; out.fin_res = bnrm2; out.status = TFS_OK; out.true_res = 0;
+            }
+        }
+        __syncthreads();
+        if (L.done) return;
+    }
+    {
+        double e2, rz;
+        batch_true_residual<METHOD, VT>(S, gtid, stride, e2, rz);
+        if (dic) rz = (double)batch_sweeps<VT, double>(S, gtid, stride, cl);
+        const double a2[2] = {e2, rz};
+        double v2[2];
+        cluster_sum<2>(a2, v2, s_part, parity, cl);
+        if (lead) {
+            const double err = sqrt(v2[0]);
+            L.err = L.ini = L.r_true = err;
+            L.rho = v2[1];
+            L.true_res = 1;
+            L.status = TFS_OK;
+            L.niter_out = L.early = 0;
+            bool stop = false;
+            if (!(err <= DBL_MAX)) { L.status = TFS_ERR_NONFINITE; L.niter_out = (S.niter_max > 0 ? S.niter_max : 0) + 1; stop = true; }
+            else if (err < S.tol) { L.early = 2; stop = true; }
+            else if (S.niter_max <= 0) { L.niter_out = 1; stop = true; }
+            L.done = stop;
+            L.beta = 0.0;
+        }
+        __syncthreads();
+    }
+
+    for (int iter = 1; !L.done; iter++) {
+        // p = z + beta p (Cg.f90:114-123; both directions for BiCG).
+        {
+            const VT betaT = (VT)L.beta;
+            const VT *const z = W.z, *const z2 = W.z2;
+            VT *const p = W.p, *const p2 = W.p2;
+            for (int i0 = gtid; i0 < n_int; i0 += 2 * stride) {
+                const int i1 = i0 + stride;
+                const bool ok1 = i1 < n_int;
+                // z past L1: with DIC other threads of the cluster wrote it
+                const VT z0 = __ldcg(z + i0), p0 = p[i0], z1 = ok1 ? __ldcg(z + i1) : (VT)0, p1 = ok1 ? p[i1] : (VT)0;
+                VT a0 = (VT)0, b0 = (VT)0, a1 = (VT)0, b1 = (VT)0;
+                if (METHOD == 1) {
+                    a0 = z2[i0]; b0 = p2[i0];
+                    if (ok1) { a1 = z2[i1]; b1 = p2[i1]; }
+                }
+                p[i0] = iter == 1 ? z0 : z0 + betaT * p0;
+                if (METHOD == 1) p2[i0] = iter == 1 ? a0 : a0 + betaT * b0;
+                if (ok1) {
+                    p[i1] = iter == 1 ? z1 : z1 + betaT * p1;
+                    if (METHOD == 1) p2[i1] = iter == 1 ? a1 : a1 + betaT * b1;
+                }
+            }
+        }
+        cl.sync();
+        // q = A p and alpha (Cg.f90:128-153 / Bicg.f90:136-165).
+        {
+            AccT pq = (AccT)0;
+            const SellDev A = S.A;
+            const VT *const val = batch_val<VT>(S), *const p = W.p;
+            VT *const q = W.q;
+            if (METHOD == 1) {
+                const VT *const p2 = W.p2;
+                VT *const q2 = W.q2;
+                for (int i = gtid; i < n_int; i += stride) {
+                    const RowGeom g = row_geom(A, i);
+                    VT s1 = (VT)0, s2 = (VT)0;
+                    row_accum2<false, VT, VT, VT>(s1, s2, A.col, val, p, p2, g.off, 0, g.len);
+                    q[i] = s1;
+                    q2[i] = s2;
+                    pq = acc_fma(p2[i], s1, pq);
+                }
+            } else {
+                batch_spmv<VT, AccT>(A, val, p, q, pq, n_int, gtid, stride);
+            }
+            const AccT a1[1] = {pq};
+            double v1[1];
+            cluster_sum<1, AccT>(a1, v1, s_part, parity, cl);
+            if (lead) L.alfa = L.rho / v1[0];
+            __syncthreads();
+        }
+        // x (or e) += alpha p, r -= alpha q, z = M^-1 r, ||r||, next rho.
+        {
+            const double alfa = L.alfa;
+            const VT alfaT = (VT)alfa;
+            AccT e2a = (AccT)0, rza = (AccT)0;
+            VT *const r = W.r, *const z = W.z, *const r2 = W.r2, *const z2 = W.z2;
+            const VT *const p = W.p, *const q = W.q, *const q2 = W.q2, *const d = W.d;
+            double *const x = S.V.x;
+            float *const e = S.F.e;
+            if (METHOD == 1) {
+                for (int i = gtid; i < n_int; i += stride) {
+                    if (MIXED) e[i] = fmaf((float)alfaT, (float)p[i], e[i]);
+                    else x[i] = x[i] + alfa * (double)p[i];
+                    const VT r1 = r[i] - alfaT * q[i];
+                    r[i] = r1;
+                    const VT dT = d[i];
+                    const VT z1 = r1 / dT;
+                    z[i] = z1;
+                    e2a = acc_fma(r1, r1, e2a);
+                    const VT rs = r2[i] - alfaT * q2[i];
+                    r2[i] = rs;
+                    z2[i] = rs / dT;
+                    rza = acc_fma(z1, rs, rza);
+                }
+            } else {
+                for (int i0 = gtid; i0 < n_int; i0 += 4 * stride) {
+                    VT pv[4], rv[4], qv[4], dv[4];
+                    double xv[4];
+                    float ev[4];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const int i = i0 + k * stride < n_int ? i0 + k * stride : i0;
+                        pv[k] = p[i]; rv[k] = r[i]; qv[k] = q[i];
+                        if (!dic) dv[k] = d[i];
+                        if (MIXED) ev[k] = e[i]; else xv[k] = x[i];
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const int i = i0 + k * stride;
+                        if (i >= n_int) continue;
+                        if (MIXED) e[i] = fmaf((float)alfaT, (float)pv[k], ev[k]);
+                        else x[i] = xv[k] + alfa * (double)pv[k];
+                        const VT r1 = rv[k] - alfaT * qv[k];
+                        r[i] = r1;
+                        e2a = acc_fma(r1, r1, e2a);
+                        if (dic) continue;
+                        const VT z1 = r1 / dv[k];
+                        z[i] = z1;
+                        rza = acc_fma(r1, z1, rza);
+                    }
+                }
+            }
+            if (dic) rza = batch_sweeps<VT, AccT>(S, gtid, stride, cl);
+            const AccT a3[2] = {e2a, rza};
+            double v3[2];
+            cluster_sum<2, AccT>(a3, v3, s_part, parity, cl);
+            if (lead) {
+                const double est = sqrt(v3[0]);
+                L.err = est;
+                L.rho_old = L.rho;
+                L.rho = v3[1];
+                L.need = MIXED && (!(est <= DBL_MAX) || est < S.tol || est < 0.1 * L.r_true || iter >= S.niter_max);
+            }
+        }
+        if (MIXED) __syncthreads();
+        if (MIXED && L.need) {
+            {
+                double *const x = S.V.x;
+                float *const e = S.F.e;
+                for (int i = gtid; i < n_int; i += stride) {
+                    x[i] = x[i] + (double)e[i];
+                    e[i] = 0.f;
+                }
             }
             cl.sync();
-            true_residual(false, e2, rz);
-            if (dic) {
-                cl.sync();
-                rz = (double)batch_dic_apply<VT, double>(A, valT, MIXED ? (const VT *)F.d : (const VT *)V.d, W.r,
-                                                         yT, W.z, S.lvl_begin, S.n_levels, gtid, stride, cl);
-            }
+            double e2, rz;
+            batch_true_residual<METHOD, VT>(S, gtid, stride, e2, rz);
+            if (dic) rz = (double)batch_sweeps<VT, double>(S, gtid, stride, cl);
             const double a4[2] = {e2, rz};
             double v4[2];
             cluster_sum<2>(a4, v4, s_part, parity, cl);
-            est = sqrt(v4[0]);
-            rho_next = v4[1];
-            r_true = est;
-            true_res++;
+            if (lead) {
+                L.r_true = L.err = sqrt(v4[0]);
+                L.rho = v4[1];
+                L.true_res++;
+            }
         }
-        err = est;
-        if (!(err <= DBL_MAX)) { status = TFS_ERR_NONFINITE; niter_out = (niter_max > 0 ? niter_max : 0) + 1; done = true; }
-        else if (err < tol) { niter_out = iter; done = true; }
-        else if (iter >= niter_max) { niter_out = iter + 1; done = true; }
-        else { iter++; rho_old = rho; rho = rho_next; }
+        if (lead) {
+            bool stop = true;
+            if (!(L.err <= DBL_MAX)) { L.status = TFS_ERR_NONFINITE; L.niter_out = (S.niter_max > 0 ? S.niter_max : 0) + 1; }
+            else if (L.err < S.tol) L.niter_out = iter;
+            else if (iter >= S.niter_max) L.niter_out = iter + 1;
+            else {
+                stop = false;
+                L.beta = L.rho / L.rho_old;
+            }
+            L.done = stop;
+        }
+        __syncthreads();
     }
     cl.sync();
     // x and r1 back to natural order.
-    for (int i = gtid; i < n_int; i += stride) {
-        int o = __ldg(S.perm + i);
-        if (o >= 0) { S.x[o] = V.x[i]; S.r_out[o] = V.r[i]; }
+    {
+        const int *const perm = S.perm;
+        double *const xo = S.x, *const ro = S.r_out;
+        const double *const x = S.V.x, *const r = S.V.r;
+        for (int i = gtid; i < n_int; i += stride) {
+            const int o = __ldg(perm + i);
+            if (o >= 0) { xo[o] = x[i]; ro[o] = r[i]; }
+        }
     }
-    if (cl.block_rank() == 0 && threadIdx.x == 0) {
-        S.niter_out = niter_out; S.status = status; S.early = early; S.true_res = true_res;
-        S.ini_res = ini; S.fin_res = err;
+    if (cl.block_rank() == 0 && lead) {
+        out.niter_out = L.niter_out; out.status = L.status; out.early = L.early; out.true_res = L.true_res;
+        out.ini_res = L.ini; out.fin_res = L.err;
     }
 }
 
@@ -487,13 +612,15 @@ __global__ void k_batch_gather(BatchSys *sys, BatchCtl *ctl, int mixed)
     }
 }
 
-template <int METHOD, typename VT>
-__global__ void __launch_bounds__(TFS_BATCH_MAX_TPB, TFS_BATCH_MIN_BLOCKS)
+template <int METHOD, typename VT, int PER_SM>
+__global__ void __launch_bounds__(TFS_BATCH_MAX_TPB, PER_SM)
 k_batch(BatchSys *sys, const int *order, int n_sys, BatchCtl *ctl)
 {
     cg::cluster_group cl = cg::this_cluster();
     __shared__ double s_part[2][4];
     __shared__ int s_sys;
+    __shared__ BatchSys s_S;
+    __shared__ BatchLead s_L;
     int parity = 0;
     for (;;) {
         if (cl.block_rank() == 0 && threadIdx.x == 0) s_sys = (int)atomicAdd(&ctl->head, 1u);
@@ -501,7 +628,11 @@ k_batch(BatchSys *sys, const int *order, int n_sys, BatchCtl *ctl)
         const int q = *cl.map_shared_rank(&s_sys, 0);
         cl.sync();   // every CTA has read rank 0's s_sys before it changes
         if (q >= n_sys) break;
-        batch_solve_one<METHOD, VT>(sys[order[q]], cl, s_part, parity);
+        BatchSys &S = sys[order[q]];
+        for (int k = threadIdx.x; k < (int)(sizeof(BatchSys) / 8); k += blockDim.x)
+            ((unsigned long long *)&s_S)[k] = ((const unsigned long long *)&S)[k];
+        __syncthreads();
+        batch_solve_one<METHOD, VT>(s_S, S, s_L, cl, s_part, parity);
         cl.sync();
     }
 }

@@ -1489,10 +1489,17 @@ static void l2_window_nodes(cudaGraph_t g, const cudaAccessPolicyWindow &w)
     }
 }
 
-#ifndef TFS_BODY_ITERATIONS
 #define TFS_BODY_ITERATIONS 4
-#endif
-#define TFS_BODY_KERNELS 10
+
+// Iterations of a loop body: TFS_BODY_ITERATIONS unless the sweeps are
+// launched level by level.
+static int body_iterations(const tfs_handle *h, int method, int prec)
+{
+    if (prec != 2) return TFS_BODY_ITERATIONS;
+    const bool mixed = h->precision == TFS_MIXED;
+    const bool few = mixed ? use_tiles<float>(h) || dic_block_kind<float>(h) : use_tiles<double>(h) || dic_block_kind<double>(h);
+    return few && method != TFS_BICG ? TFS_BODY_ITERATIONS : 1;   // (the literal BiCG sweeps two vectors by levels)
+}
 
 static int build_graph(tfs_handle *h, int method, int prec, GraphEntry &ge)
 {
@@ -1535,11 +1542,15 @@ static int build_graph(tfs_handle *h, int method, int prec, GraphEntry &ge)
     e = cudaStreamBeginCaptureToGraph(h->stream2, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return fail(e, "begin body capture");
     // A body of few kernels holds TFS_BODY_ITERATIONS iterations: going round
-    // the loop costs 4 to 5 us (a 32^3 diagonal CG iteration 21.2 -> 17.8 us,
-    // a 64^3 DIC-CG iteration 55.3 -> 51.9 mixed).  Kernels past the end of
+    // the loop costs 4 to 5 us (a 32^3 diagonal CG iteration 21.2 -> 17.4 us,
+    // a 64^3 DIC-CG iteration 55.3 -> 51.2 mixed).  Kernels past the end of
     // the solve return at once; a body of many (level kernels) would lose
-    // more to those than it gains.
-    for (int k = 0; k < TFS_BODY_ITERATIONS && !rc && (k == 0 || ge.body_kernels <= TFS_BODY_KERNELS); k++) {
+    // more to those than it gains.  (The mixed solves' true-residual step
+    // stays with every iteration: once a body it saved two idle kernels, 4 us,
+    // an iteration of a slow solve, but a fast one, which asks for it every
+    // iteration or two, then leaves most of each body idle.)
+    const int reps = body_iterations(h, method, prec);
+    for (int k = 0; k < reps && !rc; k++) {
         if (h->precision == TFS_MIXED) rc = tfs_mixed_body(h, h->stream2, method, prec, cond, &ge.body_kernels);
         else rc = launch_body(h, h->stream2, method, prec, cond, &ge.body_kernels);
     }
@@ -2301,7 +2312,9 @@ extern "C" int tfs_batch_configure(tfs_batch *b, int cluster_size, int threads_p
 template <int METHOD, typename VT>
 static int launch_batch_kernel(tfs_batch *b)
 {
-    auto kernel = k_batch<METHOD, VT>;
+    auto kernel = k_batch<METHOD, VT, 1>;
+    if constexpr (sizeof(VT) == 4)
+        if ((int64_t)b->n * b->cluster > (int64_t)TFS_BATCH_ROOMY * b->hs[0]->sm_count) kernel = k_batch<METHOD, VT, 2>;
     if (b->cluster > 8) CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
