@@ -1327,25 +1327,24 @@ static int tfs_mixed_body(tfs_handle *h, cudaStream_t s, int method, int prec,
             *count += 5;
         }
     } else {
+        const int n4 = h->n_int / 4, G4 = h->grid_vec4;
+        const bool pv = h->use_pdl && h->pdl_vec;
+        const DevState *st = h->st;
         if (prec == 2) {
-            k_mx_cgs_u<false><<<G, T, 0, s>>>(nc, F, h->st);
+            launch_ex(pv, k_mx_cgs_u4<false>, G4, T, s, n4, F, st);
             if ((rc = launch_sweeps<float>(h, s, 1, F.u2, nullptr, F.y, nullptr, F.p2, nullptr, count))) return rc;
-            k_mx_spmv_v<<<GS, T, 0, s>>>(A, v32, F, h->st, h->part);
-            k_mx_cgs_q<false><<<G, T, 0, s>>>(nc, F, h->st);
+            launch_ex(pv, k_mx_spmv_v, GS, T, s, A, v32, F, h->st, h->part);
+            launch_ex(pv, k_mx_cgs_q4<false>, G4, T, s, n4, F, st);
             if ((rc = launch_sweeps<float>(h, s, 1, F.w, nullptr, F.y, nullptr, F.p, nullptr, count))) return rc;
-            k_mx_cgs_spmv_r<<<GS, T, 0, s>>>(A, v32, V, F, h->st, h->part);
-            k_mx_fold<<<G, T, 0, s>>>(nc, V, F, h->st);
-            k_mx_true<2, false><<<G, T, 0, s>>>(A, h->val, V, F, h->st, h->part, prec, cond);
-            *count += 6;
         } else {
-            k_mx_cgs_u<true><<<G, T, 0, s>>>(nc, F, h->st);
-            k_mx_spmv_v<<<GS, T, 0, s>>>(A, v32, F, h->st, h->part);
-            k_mx_cgs_q<true><<<G, T, 0, s>>>(nc, F, h->st);
-            k_mx_cgs_spmv_r<<<GS, T, 0, s>>>(A, v32, V, F, h->st, h->part);
-            k_mx_fold<<<G, T, 0, s>>>(nc, V, F, h->st);
-            k_mx_true<2, false><<<G, T, 0, s>>>(A, h->val, V, F, h->st, h->part, prec, cond);
-            *count += 6;
+            launch_ex(pv, k_mx_cgs_u4<true>, G4, T, s, n4, F, st);
+            launch_ex(pv, k_mx_spmv_v, GS, T, s, A, v32, F, h->st, h->part);
+            launch_ex(pv, k_mx_cgs_q4<true>, G4, T, s, n4, F, st);
         }
+        launch_ex(pv, k_mx_cgs_spmv_r, GS, T, s, A, v32, V, F, h->st, h->part);
+        launch_ex(pv, k_mx_fold4, G4, T, s, n4, V, F, st);
+        launch_ex(pv, k_mx_true<2, false>, G, T, s, A, (const double *)h->val, V, F, h->st, h->part, prec, cond, 0);
+        *count += 6;
     }
     CKL("mixed body launch");
     return TFS_OK;
@@ -1408,21 +1407,22 @@ static int launch_body(tfs_handle *h, cudaStream_t s, int method, int prec,
             *count += 3;
         }
     } else {
+        const bool pv = h->use_pdl && h->pdl_vec;
+        const DevState *st = h->st;
+        const double *val = h->val;
         if (prec == 2) {
-            k_cgs_u<false><<<G, T, 0, s>>>(nc, V, h->st);
+            launch_ex(pv, k_cgs_u<false>, G, T, s, nc, V, st);
             if ((rc = launch_sweeps<double>(h, s, 1, V.u2, nullptr, V.y, nullptr, V.p2, nullptr, count))) return rc;
-            k_spmv_v<<<GS, T, 0, s>>>(A, h->val, V, h->st, h->part);
-            k_cgs_q<false><<<G, T, 0, s>>>(nc, V, h->st);
+            launch_ex(pv, k_spmv_v, GS, T, s, A, val, V, h->st, h->part);
+            launch_ex(pv, k_cgs_q<false>, G, T, s, nc, V, st);
             if ((rc = launch_sweeps<double>(h, s, 1, V.w, nullptr, V.y, nullptr, V.p, nullptr, count))) return rc;
-            k_cgs_spmv_r<<<GS, T, 0, s>>>(A, h->val, V, h->st, h->part, cond);
-            *count += 4;
         } else {
-            k_cgs_u<true><<<G, T, 0, s>>>(nc, V, h->st);
-            k_spmv_v<<<GS, T, 0, s>>>(A, h->val, V, h->st, h->part);
-            k_cgs_q<true><<<G, T, 0, s>>>(nc, V, h->st);
-            k_cgs_spmv_r<<<GS, T, 0, s>>>(A, h->val, V, h->st, h->part, cond);
-            *count += 4;
+            launch_ex(pv, k_cgs_u<true>, G, T, s, nc, V, st);
+            launch_ex(pv, k_spmv_v, GS, T, s, A, val, V, h->st, h->part);
+            launch_ex(pv, k_cgs_q<true>, G, T, s, nc, V, st);
         }
+        launch_ex(pv, k_cgs_spmv_r, GS, T, s, A, val, V, h->st, h->part, cond);
+        *count += 4;
     }
     CKL("body launch");
     return TFS_OK;

@@ -55,12 +55,20 @@ k_mx_true(SellDev A, const double *__restrict__ val, Vec64 V, Vec32 F, DevState 
     if (blockIdx.x == 0 && threadIdx.x == 0) st->t_spmv0 = gtimer();
     const bool fused = (METHOD == 2) || prec != 2;
     double e2 = 0.0, rz = 0.0;
-    for (int c = blockIdx.x; c < A.n_chunks; c += gridDim.x) {
-        int i = c * TFS_TPB + threadIdx.x;
+    struct Row {
         double b;
-        if (INIT) { b = V.r[i]; V.u1[i] = b; F.e[i] = 0.f; } else b = V.u1[i];
-        RowGeom g = row_geom(A, i);
-        double r = row_accum<true, double, double, double, TFS_SPMV_NC>(b, A.col, val, V.x, g.off, 0, g.len);
+        float d, r2;
+    };
+    auto pre = [&](int i) {
+        Row o;
+        o.b = INIT ? V.r[i] : V.u1[i];
+        o.d = METHOD != 2 && fused ? F.d[i] : 0.f;
+        o.r2 = METHOD == 2 && !INIT ? F.r2[i] : 0.f;
+        return o;
+    };
+    auto first = [](const Row &o) { return o.b; };
+    spmv_rows<true>(A, val, (const double *)V.x, pre, first, [&](int i, const Row &o, double r) {
+        if (INIT) { V.u1[i] = o.b; F.e[i] = 0.f; }
         V.r[i] = r;
         float r32 = (float)r;
         F.r[i] = r32;
@@ -72,9 +80,9 @@ k_mx_true(SellDev A, const double *__restrict__ val, Vec64 V, Vec32 F, DevState 
         // resets it together with r1; CGS keeps its initial shadow.
         if (METHOD == 1 || (INIT && METHOD == 2)) F.r2[i] = r32;
         e2 = fma(r, r, e2);
-        if (METHOD == 2) rz = fma((double)r32, (double)F.r2[i], rz);
+        if (METHOD == 2) rz = fma((double)r32, (double)(INIT ? r32 : o.r2), rz);
         else if (fused) {
-            float d32 = F.d[i], z = r32 / d32;
+            float z = r32 / o.d;
             F.z[i] = z;
             if (METHOD == 0) rz = fma((double)r32, (double)z, rz);
             else {
@@ -82,7 +90,7 @@ k_mx_true(SellDev A, const double *__restrict__ val, Vec64 V, Vec32 F, DevState 
                 rz = fma((double)z, (double)r32, rz);
             }
         }
-    }
+    });
     double v[2] = {e2, rz};
     if (grid_reduce<2>(v, part, &st->counter)) {
         double err = sqrt(v[0]);
@@ -530,40 +538,50 @@ k_mx_bicg_update(int n_chunks, Vec64 V, Vec32 F, DevState *st, double *part)
 
 // --------------------------------------------------------------- CGS
 
+// The CGS kernels are PDL-chained: each waits for its predecessor before it
+// reads anything.  k_mx_cgs_u4 and k_mx_cgs_q4 let their successor launch
+// early only without DIC, whose level kernels read their right-hand side
+// before their own wait.  16-byte loads, four rows a step, as the CG vector
+// kernels.
 template <bool FUSEDP>
-__global__ void __launch_bounds__(TFS_TPB) k_mx_cgs_u(int n_chunks, Vec32 F, const DevState *st)
+__global__ void __launch_bounds__(TFS_TPB) k_mx_cgs_u4(int n4, Vec32 F, const DevState *st)
 {
-    if (st->done || st->need_true) return;
+    cudaGridDependencySynchronize();
+    if (FUSEDP) cudaTriggerProgrammaticLaunchCompletion();
+    const bool stop = (st->done | st->need_true) != 0;
     const int it = st->iter;
     const float beta = it == 1 ? 0.f : st->beta32;
-    for (int c = blockIdx.x; c < n_chunks; c += gridDim.x) {
-        int i = c * TFS_TPB + threadIdx.x;
-        float u1, u2;
-        if (it == 1) { u1 = F.r[i]; u2 = u1; }
-        else {
-            float q1 = F.q[i];
-            u1 = F.r[i] + beta * q1;
-            u2 = u1 + beta * (q1 + beta * F.u2[i]);
-        }
-        F.u1[i] = u1;
-        F.u2[i] = u2;
-        if (FUSEDP) F.p2[i] = u2 / F.d[i];
+    const float4 *r4 = (const float4 *)F.r, *q4 = (const float4 *)F.q, *d4 = (const float4 *)F.d;
+    float4 *u4 = (float4 *)F.u1, *v4 = (float4 *)F.u2, *p4 = (float4 *)F.p2;
+    auto u1_of = [&](float r, float q) { return it == 1 ? r : r + beta * q; };
+    auto u2_of = [&](float u, float q, float v) { return it == 1 ? u : u + beta * (q + beta * v); };
+    for (int v = blockIdx.x * TFS_TPB + threadIdx.x; v < n4; v += gridDim.x * TFS_TPB) {
+        const float4 r = r4[v], q = q4[v], o = v4[v];
+        float4 d;
+        if (FUSEDP) d = d4[v];
+        if (stop) return;
+        const float4 u = make_float4(u1_of(r.x, q.x), u1_of(r.y, q.y), u1_of(r.z, q.z), u1_of(r.w, q.w));
+        const float4 w = make_float4(u2_of(u.x, q.x, o.x), u2_of(u.y, q.y, o.y), u2_of(u.z, q.z, o.z), u2_of(u.w, q.w, o.w));
+        u4[v] = u;
+        v4[v] = w;
+        if (FUSEDP) p4[v] = make_float4(w.x / d.x, w.y / d.y, w.z / d.z, w.w / d.w);
     }
 }
 
 __global__ void __launch_bounds__(TFS_TPB)
 k_mx_spmv_v(SellDev A, const float *__restrict__ val, Vec32 F, DevState *st, double *part)
 {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
     if (st->done || st->need_true) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) st->t_spmv0 = gtimer();
     float acc = 0.f;
-    for (int c = blockIdx.x; c < A.n_chunks; c += gridDim.x) {
-        int i = c * TFS_TPB + threadIdx.x;
-        RowGeom g = row_geom(A, i);
-        float s = row_accum<false, float, float, float, TFS_SPMV_NC>(0.f, A.col, val, F.p2, g.off, 0, g.len);
+    auto pre = [&](int i) { return Row1<float>{F.r2[i]}; };
+    auto first = [](const Row1<float> &) { return 0.f; };
+    spmv_rows<false>(A, val, (const float *)F.p2, pre, first, [&](int i, const Row1<float> &o, float s) {
         F.v2[i] = s;
-        acc = fmaf(F.r2[i], s, acc);
-    }
+        acc = fmaf(o.a, s, acc);
+    });
     const float av[1] = {acc};
     double v[1];
     if (grid_reduce_f<1>(av, v, part, &st->counter)) {
@@ -575,18 +593,24 @@ k_mx_spmv_v(SellDev A, const float *__restrict__ val, Vec32 F, DevState *st, dou
 }
 
 template <bool FUSEDP>
-__global__ void __launch_bounds__(TFS_TPB) k_mx_cgs_q(int n_chunks, Vec32 F, const DevState *st)
+__global__ void __launch_bounds__(TFS_TPB) k_mx_cgs_q4(int n4, Vec32 F, const DevState *st)
 {
-    if (st->done || st->need_true) return;
-    const float alfa32 = (float)st->alpha;
-    for (int c = blockIdx.x; c < n_chunks; c += gridDim.x) {
-        int i = c * TFS_TPB + threadIdx.x;
-        float u1 = F.u1[i];
-        float q1 = u1 - alfa32 * F.v2[i];
-        F.q[i] = q1;
-        float w = u1 + q1;
-        if (FUSEDP) F.p[i] = w / F.d[i];
-        else F.w[i] = w;
+    cudaGridDependencySynchronize();
+    if (FUSEDP) cudaTriggerProgrammaticLaunchCompletion();
+    const bool stop = (st->done | st->need_true) != 0;
+    const float a = (float)st->alpha;
+    const float4 *u4 = (const float4 *)F.u1, *v4 = (const float4 *)F.v2, *d4 = (const float4 *)F.d;
+    float4 *q4 = (float4 *)F.q, *w4 = (float4 *)F.w, *p4 = (float4 *)F.p;
+    for (int v = blockIdx.x * TFS_TPB + threadIdx.x; v < n4; v += gridDim.x * TFS_TPB) {
+        const float4 u = u4[v], t = v4[v];
+        float4 d;
+        if (FUSEDP) d = d4[v];
+        if (stop) return;
+        const float4 q = make_float4(u.x - a * t.x, u.y - a * t.y, u.z - a * t.z, u.w - a * t.w);
+        const float4 w = make_float4(u.x + q.x, u.y + q.y, u.z + q.z, u.w + q.w);
+        q4[v] = q;
+        if (FUSEDP) p4[v] = make_float4(w.x / d.x, w.y / d.y, w.z / d.z, w.w / d.w);
+        else w4[v] = w;
     }
 }
 
@@ -594,21 +618,22 @@ __global__ void __launch_bounds__(TFS_TPB)
 k_mx_cgs_spmv_r(SellDev A, const float *__restrict__ val, Vec64 V, Vec32 F, DevState *st,
                 double *part)
 {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
     if (st->done || st->need_true) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) st->t_spmv0 = gtimer();
     const double alfa = st->alpha;
     const float alfa32 = (float)alfa;
     float e2 = 0.f, rr = 0.f;
-    for (int c = blockIdx.x; c < A.n_chunks; c += gridDim.x) {
-        int i = c * TFS_TPB + threadIdx.x;
-        F.e[i] = fmaf(alfa32, F.p[i], F.e[i]);
-        RowGeom g = row_geom(A, i);
-        float q2 = row_accum<false, float, float, float, TFS_SPMV_NC>(0.f, A.col, val, F.p, g.off, 0, g.len);
-        float r1 = fmaf(-alfa32, q2, F.r[i]);
+    auto pre = [&](int i) { return Row4<float>{F.p[i], F.e[i], F.r[i], F.r2[i]}; };
+    auto first = [](const Row4<float> &) { return 0.f; };
+    spmv_rows<false>(A, val, (const float *)F.p, pre, first, [&](int i, const Row4<float> &o, float q2) {
+        F.e[i] = fmaf(alfa32, o.p, o.x);
+        float r1 = fmaf(-alfa32, q2, o.r);
         F.r[i] = r1;
         e2 = fmaf(r1, r1, e2);
-        rr = fmaf(r1, F.r2[i], rr);
-    }
+        rr = fmaf(r1, o.r2, rr);
+    });
     const float av[2] = {e2, rr};
     double v[2];
     if (grid_reduce_f<2>(av, v, part, &st->counter)) {

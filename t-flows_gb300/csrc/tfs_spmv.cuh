@@ -22,44 +22,6 @@
 
 namespace tfs {
 
-#ifndef TFS_SPMV_NOALLOC
-#define TFS_SPMV_NOALLOC 1
-#endif
-// Read-once matrix stream (values, column indices, geometry) loaded without
-// allocating in L1, so that L1 holds the gathered p: binary32 SpMV 31.2
-// against 32.8 us on the 128^3 system (binary64 unchanged, 73.8 us).
-__device__ __forceinline__ int ld_stream(const int *a)
-{
-    int v;
-    if (TFS_SPMV_NOALLOC) asm("ld.global.nc.L1::no_allocate.b32 %0, [%1];" : "=r"(v) : "l"(a));
-    else v = __ldg(a);
-    return v;
-}
-__device__ __forceinline__ uint32_t ld_stream(const uint32_t *a)
-{
-    uint32_t v;
-    if (TFS_SPMV_NOALLOC) asm("ld.global.nc.L1::no_allocate.b32 %0, [%1];" : "=r"(v) : "l"(a));
-    else v = __ldg(a);
-    return v;
-}
-__device__ __forceinline__ float ld_stream(const float *a)
-{
-    float v;
-    if (TFS_SPMV_NOALLOC) asm("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(a));
-    else v = __ldg(a);
-    return v;
-}
-__device__ __forceinline__ double ld_stream(const double *a)
-{
-    double v;
-    if (TFS_SPMV_NOALLOC) asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(a));
-    else v = __ldg(a);
-    return v;
-}
-
-__device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
-__device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
-
 // q = A p; (p, q); alpha, software-pipelined over the thread's rows c *
 // 256 + tid, c = blockIdx.x, blockIdx.x + gridDim.x, ... (the direct
 // kernels' rows and order).  W: the matrix's uniform slice width.
