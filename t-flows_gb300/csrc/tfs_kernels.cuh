@@ -1103,9 +1103,13 @@ k_spmv_pq(SellDev A, const double *__restrict__ val, const double *__restrict__ 
 }
 
 // x += alpha p, r -= alpha q (Cg.f90:159-162), ||r|| and the test; with
-// FUSED also rho of the next iteration, (r, r/d).
+// FUSED also rho of the next iteration, (r, r/d).  Four blocks an SM (at most
+// 64 registers): the grid of eight an SM is then two full waves, not the
+// three, the last one short, of the 73 to 78 registers the compiler takes
+// freely (a 128^3 iteration, diagonal 168 -> 158 us, DIC 293 -> 285; capped
+// for eight blocks, with spills, 171 and 297).
 template <bool FUSED>
-__global__ void __launch_bounds__(TFS_TPB)
+__global__ void __launch_bounds__(TFS_TPB, 4)
 k_cg_update(int n_chunks, Vec64 V, DevState *st, double *part, cudaGraphConditionalHandle cond,
             int l0_rows = 0)
 {
