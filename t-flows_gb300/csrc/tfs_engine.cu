@@ -24,6 +24,7 @@
 #include "tfs_kernels.cuh"
 #include "tfs_mixed.cuh"
 #include "tfs_spmv.cuh"
+#include "tfs_cg_resident.cuh"
 #include "tfs_dic_block.cuh"
 #include "tfs_dic_tiles.cuh"
 
@@ -278,6 +279,58 @@ static void launch_spmv_pq(tfs_handle *h, cudaStream_t s, bool mixed, bool pdl =
     } else {
         k_spmv_pq<<<VG, TFS_TPB, 0, s>>>(A, h->val, h->v.p, h->v.q, h->st, h->part);
     }
+}
+
+// The part buffer: TFS_NPART partials a block, then (systems that may solve
+// by k_cg_resident) that kernel's slots and exchange number.
+#define TFS_RESIDENT_CHUNKS 512
+static size_t part_slots(const tfs_handle *h) { return TFS_NPART * (size_t)h->n_chunks + 64; }
+static size_t part_doubles(const tfs_handle *h)
+{
+    return part_slots(h) + (h->n_chunks <= TFS_RESIDENT_CHUNKS ? 6 * (size_t)h->n_chunks + 2 : 0);
+}
+
+template <int W>
+static cudaError_t launch_cg_resident(const tfs_handle *h, cudaStream_t s)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)h->n_chunks);
+    cfg.blockDim = dim3(TFS_TPB);
+    cfg.stream = s;
+    // One block per multiprocessor while there are enough: two on one share
+    // its binary64 pipe, and every other block waits for them.
+    if (h->n_chunks <= h->sm_count) {
+        int smem = 0;
+        cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, h->device);
+        cfg.dynamicSmemBytes = (size_t)smem / 2;
+        const cudaError_t e = cudaFuncSetAttribute(k_cg_resident<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)cfg.dynamicSmemBytes);
+        if (e != cudaSuccess) return e;
+    }
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    CgSlot *slots = (CgSlot *)(h->part + part_slots(h));
+    return cudaLaunchKernelEx(&cfg, k_cg_resident<W>, sell_of(h), (const double *)h->val, h->v, h->st, slots,
+                              (unsigned long long *)(slots + 3 * (size_t)h->n_chunks));
+}
+
+// Whether the CG loop runs as k_cg_resident: binary64 without DIC, every
+// block resident, and not of a server, whose other requests' kernels share
+// the multiprocessors.  (Faster than the kernels of an iteration at every
+// size it can take.)
+static bool use_cg_resident(const tfs_handle *h, int method, int prec)
+{
+    if (method != TFS_CG || prec == 2 || h->precision == TFS_MIXED || h->no_resident) return false;
+    if (h->row_max > 8 || h->n_chunks > TFS_RESIDENT_CHUNKS) return false;
+    if (h->grid != h->n_chunks || h->grid_spmv != h->n_chunks || h->tile_room != INT64_MAX) return false;
+    int per_sm = 0;
+    const cudaError_t e = h->row_max <= 4
+        ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg_resident<4>, TFS_TPB, 0)
+        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg_resident<8>, TFS_TPB, 0);
+    return e == cudaSuccess && h->n_chunks <= per_sm * h->sm_count;
 }
 
 static uint64_t fingerprint(int32_t n, int32_t nnz, const int32_t *row1, const int32_t *col1,
@@ -583,6 +636,7 @@ static int build_layout(tfs_handle *h, int kind)
     // widths on the 128^3 system (binary32 SpMV 39.3 against 39.5 us);
     // TFS_OPT_SELL_UNIFORM = 0 keeps per-slice widths.
     h->sell_width = 0;
+    h->row_max = wmax;
     {
         const int64_t uni = 32 * (int64_t)wmax * n_slices;
         if (h->sell_uniform && wmax > 0 && wmax <= 8 && uni <= off + off / 20 && uni <= INT32_MAX) {
@@ -626,7 +680,7 @@ static int build_layout(tfs_handle *h, int kind)
         (rc = dalloc(h, &h->rowinfo, n_int)) || (rc = dalloc(h, &h->slice_off, n_slices + 1)) ||
         (rc = dalloc(h, &h->col, nnz_pad)) || (rc = dalloc(h, &h->vmap, nnz_pad)) ||
         (rc = dalloc(h, &h->val, nnz_pad)) || (rc = dalloc(h, &h->val32, nnz_pad)) ||
-        (rc = dalloc(h, &h->part, TFS_NPART * (size_t)h->n_chunks + 64)))
+        (rc = dalloc(h, &h->part, part_doubles(h))))
         return rc;
     {
         // The tail: the levels after the last level with more than
@@ -688,7 +742,7 @@ static int build_layout(tfs_handle *h, int kind)
     CK(cudaMemcpyAsync(h->vmap, vmap.data(), sizeof(int) * (size_t)nnz_pad, cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemsetAsync(h->val, 0, sizeof(double) * (size_t)nnz_pad, h->stream));
     CK(cudaMemsetAsync(h->val32, 0, sizeof(float) * (size_t)nnz_pad, h->stream));
-    CK(cudaMemsetAsync(h->part, 0, sizeof(double) * (TFS_NPART * (size_t)h->n_chunks + 64), h->stream));
+    CK(cudaMemsetAsync(h->part, 0, sizeof(double) * part_doubles(h), h->stream));
 
     // Work vectors: 16 binary64 + 16 binary32, zero so padding rows stay zero.
     const size_t nv64 = 16, nv32 = 16;
@@ -1507,8 +1561,10 @@ static int build_graph(tfs_handle *h, int method, int prec, GraphEntry &ge)
     l2_window_streams(h, l2w);
     cudaGraph_t g = nullptr;
     CK(cudaGraphCreate(&g, 0));
-    cudaGraphConditionalHandle cond;
-    cudaError_t e = cudaGraphConditionalHandleCreate(&cond, g, 1u, cudaGraphCondAssignDefault);
+    const bool resident = use_cg_resident(h, method, prec);   // no loop in the graph
+    cudaGraphConditionalHandle cond = 0;
+    cudaError_t e = cudaSuccess;
+    if (!resident) e = cudaGraphConditionalHandleCreate(&cond, g, 1u, cudaGraphCondAssignDefault);
     if (e != cudaSuccess) { cudaGraphDestroy(g); return tfs_engine_error(e, "cudaGraphConditionalHandleCreate"); }
     int rc = TFS_OK;
     auto fail = [&](cudaError_t err, const char *what) {
@@ -1522,49 +1578,56 @@ static int build_graph(tfs_handle *h, int method, int prec, GraphEntry &ge)
     e = cudaStreamBeginCaptureToGraph(h->stream, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return fail(e, "begin capture");
     if ((rc = launch_prologue(h, h->stream, method, prec, cond, &ge.prologue_kernels))) { fail(cudaErrorUnknown, "prologue"); return rc; }
-    cudaStreamCaptureStatus cs;
-    const cudaGraphNode_t *deps = nullptr;
-    size_t ndeps = 0;
-    e = cudaStreamGetCaptureInfo(h->stream, &cs, nullptr, nullptr, &deps, nullptr, &ndeps);
-    if (e != cudaSuccess) return fail(e, "cudaStreamGetCaptureInfo");
-    cudaGraphNodeParams np = {};
-    np.type = cudaGraphNodeTypeConditional;
-    np.conditional.handle = cond;
-    np.conditional.type = cudaGraphCondTypeWhile;
-    np.conditional.size = 1;
-    cudaGraphNode_t wnode;
-    e = cudaGraphAddNode(&wnode, g, deps, nullptr, ndeps, &np);
-    if (e != cudaSuccess) return fail(e, "cudaGraphAddNode(while)");
-    cudaGraph_t body = np.conditional.phGraph_out[0];
-    e = cudaStreamUpdateCaptureDependencies(h->stream, &wnode, nullptr, 1, cudaStreamSetCaptureDependencies);
-    if (e != cudaSuccess) return fail(e, "cudaStreamUpdateCaptureDependencies");
-    // Body, captured on the second stream into the conditional node's graph.
-    e = cudaStreamBeginCaptureToGraph(h->stream2, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) return fail(e, "begin body capture");
-    // A body of few kernels holds TFS_BODY_ITERATIONS iterations: going round
-    // the loop costs 4 to 5 us (a 32^3 diagonal CG iteration 21.2 -> 17.4 us,
-    // a 64^3 DIC-CG iteration 55.3 -> 51.2 mixed).  Kernels past the end of
-    // the solve return at once; a body of many (level kernels) would lose
-    // more to those than it gains.  (The mixed solves' true-residual step
-    // stays with every iteration: once a body it saved two idle kernels, 4 us,
-    // an iteration of a slow solve, but a fast one, which asks for it every
-    // iteration or two, then leaves most of each body idle.)
-    const int reps = body_iterations(h, method, prec);
-    for (int k = 0; k < reps && !rc; k++) {
-        if (h->precision == TFS_MIXED) rc = tfs_mixed_body(h, h->stream2, method, prec, cond, &ge.body_kernels);
-        else rc = launch_body(h, h->stream2, method, prec, cond, &ge.body_kernels);
+    cudaGraph_t body = nullptr;
+    if (resident) {
+        e = h->row_max <= 4 ? launch_cg_resident<4>(h, h->stream) : launch_cg_resident<8>(h, h->stream);
+        if (e != cudaSuccess) return fail(e, "k_cg_resident");
+        ge.prologue_kernels += 1;
+    } else {
+        cudaStreamCaptureStatus cs;
+        const cudaGraphNode_t *deps = nullptr;
+        size_t ndeps = 0;
+        e = cudaStreamGetCaptureInfo(h->stream, &cs, nullptr, nullptr, &deps, nullptr, &ndeps);
+        if (e != cudaSuccess) return fail(e, "cudaStreamGetCaptureInfo");
+        cudaGraphNodeParams np = {};
+        np.type = cudaGraphNodeTypeConditional;
+        np.conditional.handle = cond;
+        np.conditional.type = cudaGraphCondTypeWhile;
+        np.conditional.size = 1;
+        cudaGraphNode_t wnode;
+        e = cudaGraphAddNode(&wnode, g, deps, nullptr, ndeps, &np);
+        if (e != cudaSuccess) return fail(e, "cudaGraphAddNode(while)");
+        body = np.conditional.phGraph_out[0];
+        e = cudaStreamUpdateCaptureDependencies(h->stream, &wnode, nullptr, 1, cudaStreamSetCaptureDependencies);
+        if (e != cudaSuccess) return fail(e, "cudaStreamUpdateCaptureDependencies");
+        // Body, captured on the second stream into the conditional node's graph.
+        e = cudaStreamBeginCaptureToGraph(h->stream2, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+        if (e != cudaSuccess) return fail(e, "begin body capture");
+        // A body of few kernels holds TFS_BODY_ITERATIONS iterations: going round
+        // the loop costs 4 to 5 us (a 32^3 diagonal CG iteration 21.2 -> 17.4 us,
+        // a 64^3 DIC-CG iteration 55.3 -> 51.2 mixed).  Kernels past the end of
+        // the solve return at once; a body of many (level kernels) would lose
+        // more to those than it gains.  (The mixed solves' true-residual step
+        // stays with every iteration: once a body it saved two idle kernels, 4 us,
+        // an iteration of a slow solve, but a fast one, which asks for it every
+        // iteration or two, then leaves most of each body idle.)
+        const int reps = body_iterations(h, method, prec);
+        for (int k = 0; k < reps && !rc; k++) {
+            if (h->precision == TFS_MIXED) rc = tfs_mixed_body(h, h->stream2, method, prec, cond, &ge.body_kernels);
+            else rc = launch_body(h, h->stream2, method, prec, cond, &ge.body_kernels);
+        }
+        if (rc) { fail(cudaErrorUnknown, "body"); return rc; }
+        cudaGraph_t btmp;
+        e = cudaStreamEndCapture(h->stream2, &btmp);
+        if (e != cudaSuccess) return fail(e, "end body capture");
     }
-    if (rc) { fail(cudaErrorUnknown, "body"); return rc; }
-    cudaGraph_t btmp;
-    e = cudaStreamEndCapture(h->stream2, &btmp);
-    if (e != cudaSuccess) return fail(e, "end body capture");
     if ((rc = launch_epilogue(h, &ge.epilogue_kernels))) { fail(cudaErrorUnknown, "epilogue"); return rc; }
     cudaGraph_t gtmp;
     e = cudaStreamEndCapture(h->stream, &gtmp);
     if (e != cudaSuccess) { cudaGraphDestroy(g); return tfs_engine_error(e, "end capture"); }
     if (l2w.num_bytes) {
         l2_window_nodes(g, l2w);
-        l2_window_nodes(body, l2w);
+        if (body) l2_window_nodes(body, l2w);
     }
     e = cudaGraphInstantiate(&ge.exec, g, 0);
     if (e != cudaSuccess) { cudaGraphDestroy(g); return tfs_engine_error(e, "cudaGraphInstantiate"); }
@@ -1614,6 +1677,12 @@ static int get_graph(tfs_handle *h, int method, int prec, GraphEntry **out)
     if (it != h->graphs.end()) { *out = &it->second; return TFS_OK; }
     GraphEntry ge;
     int rc = build_graph(h, method, prec, ge);
+    if (rc && use_cg_resident(h, method, prec)) {
+        // A driver that cannot hold a cooperative launch in a graph.
+        h->no_resident = 1;
+        ge = GraphEntry();
+        rc = build_graph(h, method, prec, ge);
+    }
     if (rc && h->use_pdl) {
         // A driver that cannot keep programmatic edges inside a conditional
         // body gets plain stream-ordered level launches instead.

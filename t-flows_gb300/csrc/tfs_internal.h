@@ -119,6 +119,8 @@ struct tfs_handle {
     int32_t n = 0, nnz = 0;
     int n_int = 0, n_chunks = 0, n_slices = 0, nnz_pad = 0, n_levels = 0;
     int sell_width = 0;                // uniform slice width (0: per-slice widths)
+    int row_max = 0;                   // entries of the longest row
+    int no_resident = 0;               // k_cg_resident could not be captured
     int spmv_kind = 0;                 // TFS_SPMV_DIRECT / _PIPE: kernel of the CG SpMV
     int grid = 0;                      // blocks of the vector kernels (grid-stride)
     int grid_spmv = 0;                 // blocks of the SpMV-type kernels
