@@ -416,7 +416,7 @@ k_rho_l0(const T *__restrict__ r, const T *__restrict__ z, int l0_rows, int n_in
         last = grid_reduce_f<1>(av, v, part, &st->counter);
     } else {
         v[0] = acc;
-        last = grid_reduce<1>(v, part, &st->counter);
+        last = grid_reduce<1, false>(v, part, &st->counter);
     }
     if (last) {
         st->rho = v[0];

@@ -276,6 +276,52 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double (*sm)[TFS_TPB 
     }
 }
 
+// The same sums, for kernels of few rows a thread: the values go through
+// shared memory and one warp adds for all eight (warp k value k).  Packed, a level of the eight warps' trees takes
+// 4, 2, 1, 1 and 1 binary64 instructions where each warp's own shuffles take
+// 8, most of their lanes idle, on the pipe that bounds these kernels.  (Not in the SpMV: 2 KB a block
+// off its L1 cost more, 69 -> 75 us binary64, 30 -> 37 binary32 at 128^3.)
+template <int NV>
+__device__ __forceinline__ void block_sum_packed(double (&v)[NV])
+{
+    static_assert(NV <= TFS_TPB / 32 && TFS_TPB == 256, "");
+    __shared__ double buf[NV][TFS_TPB], tot[NV];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < NV; k++) buf[k][threadIdx.x] = v[k];
+    __syncthreads();
+    if (warp < NV) {
+        // t[k]: lanes l and l + 16 (l = lane & 15) of warp 2 k + lane / 16
+        const double *s = buf[warp] + (lane & 16) * 2 + (lane & 15);
+        double t[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) t[k] = s[64 * k] + s[64 * k + 16];
+        // by 8: warps of t[0], t[2] in the lanes without bit 3, of t[1], t[3] in those with
+        const bool h8 = (lane & 8) != 0, h4 = (lane & 4) != 0;
+        const double x0 = __shfl_xor_sync(FULL, h8 ? t[0] : t[1], 8), x1 = __shfl_xor_sync(FULL, h8 ? t[2] : t[3], 8);
+        const double u0 = (h8 ? t[1] : t[0]) + x0, u1 = (h8 ? t[3] : t[2]) + x1;
+        // by 4: u0 without bit 2, u1 with
+        const double x2 = __shfl_xor_sync(FULL, h4 ? u0 : u1, 4);
+        double w = (h4 ? u1 : u0) + x2;
+        w = w + __shfl_xor_sync(FULL, w, 2);
+        w = w + __shfl_xor_sync(FULL, w, 1);
+        // warp q's sum lies in the lanes with bits 4, 3, 2 = bits 0, 1, 2 of q
+        double r = __shfl_sync(FULL, w, 0);
+#pragma unroll
+        for (int q = 1; q < TFS_TPB / 32; q++)
+            r = r + __shfl_sync(FULL, w, ((q & 1) << 4) | ((q & 2) << 2) | (q & 4));
+        if (NV == 1) v[0] = r;
+        else if (lane == 0) tot[warp] = r;
+    }
+    if (NV > 1) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+#pragma unroll
+            for (int k = 0; k < NV; k++) v[k] = tot[k];
+        }
+    }
+}
+
 // Sum over a warp of binary32 values, returned in binary64 by lane 0.  The
 // running sum is a binary32 pair (hi, lo) updated with Knuth's TwoSum, so it
 // carries about 48 significant bits without any binary64 instruction per
@@ -363,14 +409,15 @@ __device__ __forceinline__ bool grid_publish(double (&v)[NV], double *__restrict
     return false;
 }
 
-// Single-pass grid reduction of binary64 values (warp shuffles, then one
-// partial per block, then the last block sums the partials in block order).
-template <int NV>
+// Single-pass grid reduction of binary64 values (block sums, then one partial
+// per block, then the last block sums the partials in block order).
+template <int NV, bool PACKED = true>
 __device__ __forceinline__ bool grid_reduce(double (&v)[NV], double *__restrict__ part,
                                             unsigned int *counter)
 {
     __shared__ double sm[NV][TFS_TPB / 32];
-    block_sum<NV>(v, sm);
+    if constexpr (PACKED) block_sum_packed<NV>(v);
+    else block_sum<NV>(v, sm);
     return grid_publish<NV>(v, part, counter, sm);
 }
 
@@ -385,21 +432,25 @@ __device__ __forceinline__ bool grid_reduce_f(const float (&v)[NV], double (&out
     return grid_publish<NV>(out, part, counter, sm);
 }
 
-// Row loops of the vector kernels: four chunks per step, with every load of
-// the four rows issued before any of them is used (memory-level parallelism;
-// the stores of one row could otherwise alias the loads of the next).
-#define TFS_QUAD_BEGIN(nch)                                                   \
-    for (int _c0 = blockIdx.x; _c0 < (nch); _c0 += 4 * (int)gridDim.x) {    \
-        int _i[4];                                                           \
-        bool _ok[4];                                                         \
-        _Pragma("unroll") for (int _q = 0; _q < 4; _q++) {                   \
+// Row loops of the vector kernels: W (four) chunks per step, with every load
+// of the W rows issued before any of them is used (memory-level parallelism;
+// the stores of one row could otherwise alias the loads of the next).  Grids
+// of one or two chunks a block step by as many (step_width): the rows that a
+// step does not have would still take their turn in the binary64 pipe.
+#define TFS_STEP_BEGIN(nch, W)                                                \
+    constexpr int _w = (W);                                                   \
+    for (int _c0 = blockIdx.x; _c0 < (nch); _c0 += _w * (int)gridDim.x) {     \
+        int _i[_w];                                                          \
+        bool _ok[_w];                                                        \
+        _Pragma("unroll") for (int _q = 0; _q < _w; _q++) {                  \
             int _c = _c0 + _q * (int)gridDim.x;                              \
-            _ok[_q] = _c < (nch);                                            \
+            _ok[_q] = _w == 1 || _c < (nch);                                 \
             _i[_q] = _ok[_q] ? _c * TFS_TPB + (int)threadIdx.x : 0;          \
         }
+#define TFS_QUAD_BEGIN(nch) TFS_STEP_BEGIN(nch, 4)
 #define TFS_QLOAD(arr, ptr)                                                   \
-    _Pragma("unroll") for (int _q = 0; _q < 4; _q++) arr[_q] = (ptr)[_i[_q]];
-#define TFS_QUAD_FOR _Pragma("unroll") for (int _q = 0; _q < 4; _q++) if (_ok[_q])
+    _Pragma("unroll") for (int _q = 0; _q < _w; _q++) arr[_q] = (ptr)[_i[_q]];
+#define TFS_QUAD_FOR _Pragma("unroll") for (int _q = 0; _q < _w; _q++) if (_ok[_q])
 #define TFS_QUAD_END }
 
 __device__ __forceinline__ void set_cond(cudaGraphConditionalHandle cond, unsigned v)
@@ -1023,7 +1074,7 @@ k_sweep_tail1(SellDev A, const T *__restrict__ val, const T *d, const T *b, T *y
 }
 
 // rho after the sweeps: CG (r, z) (Cg.f90:108-112); BiCG (z1, r2) (Bicg.f90:113-117).
-template <int METHOD>
+template <int METHOD, int W>
 __global__ void __launch_bounds__(TFS_TPB)
 k_dot_rho(int n_chunks, Vec64 V, DevState *st, double *part)
 {
@@ -1033,8 +1084,8 @@ k_dot_rho(int n_chunks, Vec64 V, DevState *st, double *part)
     cudaTriggerProgrammaticLaunchCompletion();
     const bool stop = st->done != 0;
     double acc = 0.0;
-    TFS_QUAD_BEGIN(n_chunks)
-        double a[4], b[4];
+    TFS_STEP_BEGIN(n_chunks, W)
+        double a[W], b[W];
         TFS_QLOAD(a, METHOD == 0 ? V.r : V.z);
         TFS_QLOAD(b, METHOD == 0 ? V.z : V.r2);
         if (stop) return;
@@ -1056,7 +1107,7 @@ k_dot_rho(int n_chunks, Vec64 V, DevState *st, double *part)
 
 // p = z (first iteration) or z + beta p (Cg.f90:114-123); z = r/d unless the
 // DIC sweeps produced it (FROMZ).
-template <bool FROMZ>
+template <bool FROMZ, int W>
 __global__ void __launch_bounds__(TFS_TPB) k_cg_p(int n_chunks, Vec64 V, const DevState *st)
 {
     cudaGridDependencySynchronize();   // PDL secondary, as k_dot_rho
@@ -1064,10 +1115,10 @@ __global__ void __launch_bounds__(TFS_TPB) k_cg_p(int n_chunks, Vec64 V, const D
     const bool stop = st->done != 0;
     const int it = st->iter;
     const double beta = st->beta;            // rho / rho_old, published once
-    TFS_QUAD_BEGIN(n_chunks)
-        double z[4], p[4];
+    TFS_STEP_BEGIN(n_chunks, W)
+        double z[W], p[W];
         if (FROMZ) { TFS_QLOAD(z, V.z); }
-        else { double r[4], d[4]; TFS_QLOAD(r, V.r); TFS_QLOAD(d, V.d); TFS_QUAD_FOR z[_q] = r[_q] / d[_q]; }
+        else { double r[W], d[W]; TFS_QLOAD(r, V.r); TFS_QLOAD(d, V.d); TFS_QUAD_FOR z[_q] = r[_q] / d[_q]; }
         TFS_QLOAD(p, V.p);
         if (stop) return;
         TFS_QUAD_FOR V.p[_i[_q]] = it == 1 ? z[_q] : z[_q] + beta * p[_q];
@@ -1103,13 +1154,18 @@ k_spmv_pq(SellDev A, const double *__restrict__ val, const double *__restrict__ 
 }
 
 // x += alpha p, r -= alpha q (Cg.f90:159-162), ||r|| and the test; with
-// FUSED also rho of the next iteration, (r, r/d).  Four blocks an SM (at most
-// 64 registers): the grid of eight an SM is then two full waves, not the
-// three, the last one short, of the 73 to 78 registers the compiler takes
-// freely (a 128^3 iteration, diagonal 168 -> 158 us, DIC 293 -> 285; capped
-// for eight blocks, with spills, 171 and 297).
-template <bool FUSED>
-__global__ void __launch_bounds__(TFS_TPB, 4)
+// FUSED also rho of the next iteration, (r, r/d).  Grids of four chunks a
+// block and more run four blocks an SM (at most 64 registers): the grid of
+// eight an SM is then two full waves, not the three, the last one short, of
+// the 73 to 78 registers the compiler takes freely (a 128^3 iteration,
+// diagonal 168 -> 158 us, DIC 293 -> 285; capped for eight blocks, with
+// spills, 171 and 297).  Grids of one chunk a block (W = 1) run eight blocks
+// an SM, one wave.  With that, the packed block sums and no rows that a step
+// does not have, 12 us instead of 19 at 64^3 from cold caches; a 64^3
+// iteration, diagonal 45.1 -> 37.1 us, DIC 89.5 -> 78.6, a 128^3 one 158 ->
+// 153 and 285 -> 280.
+template <bool FUSED, int W>
+__global__ void __launch_bounds__(TFS_TPB, W == 1 ? 8 : W == 2 ? 6 : 4)
 k_cg_update(int n_chunks, Vec64 V, DevState *st, double *part, cudaGraphConditionalHandle cond,
             int l0_rows = 0)
 {
@@ -1119,8 +1175,8 @@ k_cg_update(int n_chunks, Vec64 V, DevState *st, double *part, cudaGraphConditio
     const bool stop = st->done != 0;
     const double alfa = st->alpha;
     double e2 = 0.0, rz = 0.0;
-    TFS_QUAD_BEGIN(n_chunks)
-        double x[4], p[4], r[4], q[4], d[4];
+    TFS_STEP_BEGIN(n_chunks, W)
+        double x[W], p[W], r[W], q[W], d[W];
         TFS_QLOAD(x, V.x); TFS_QLOAD(p, V.p); TFS_QLOAD(r, V.r); TFS_QLOAD(q, V.q);
         if (FUSED) { TFS_QLOAD(d, V.d); }
         if (stop) break;
@@ -1139,8 +1195,13 @@ k_cg_update(int n_chunks, Vec64 V, DevState *st, double *part, cudaGraphConditio
         if (blockIdx.x == 0 && threadIdx.x == 0) set_cond(cond, 0u);
         return;
     }
-    double v[2] = {e2, rz};
-    if (grid_reduce<2>(v, part, &st->counter)) finish_iteration(st, v[0], v[1], FUSED, cond);
+    if constexpr (FUSED) {
+        double v[2] = {e2, rz};
+        if (grid_reduce<2>(v, part, &st->counter)) finish_iteration(st, v[0], v[1], true, cond);
+    } else {
+        double v[1] = {e2};
+        if (grid_reduce<1>(v, part, &st->counter)) finish_iteration(st, v[0], 0.0, false, cond);
+    }
 }
 
 // -------------------------------------------------------------- BiCG body

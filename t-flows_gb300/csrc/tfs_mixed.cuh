@@ -442,7 +442,7 @@ k_sweep0_rho(SellDev A, const T *__restrict__ val, const T *d, const T *r, T *z,
         last = grid_reduce_f<1>(av, v, part, &st->counter);
     } else {
         v[0] = acc;
-        last = grid_reduce<1>(v, part, &st->counter);
+        last = grid_reduce<1, false>(v, part, &st->counter);
     }
     if (last) {
         st->rho = v[0];

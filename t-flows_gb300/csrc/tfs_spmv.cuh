@@ -24,7 +24,8 @@ namespace tfs {
 
 // q = A p; (p, q); alpha, software-pipelined over the thread's rows c *
 // 256 + tid, c = blockIdx.x, blockIdx.x + gridDim.x, ... (the direct
-// kernels' rows and order).  W: the matrix's uniform slice width.
+// kernels' rows and order).  W: the matrix's uniform slice width.  PACKED:
+// block_sum_packed (binary64).
 // Minimum resident blocks per SM asked of the compiler (register cap).
 // Unconstrained (1) is kept: on the 128^3 system the binary32 kernel runs
 // at 52 registers (4 blocks per SM) in 31.5 us; capped to 47 or 40
@@ -38,7 +39,7 @@ namespace tfs {
 #ifndef TFS_PIPE_MINB64
 #define TFS_PIPE_MINB64 1
 #endif
-template <typename VT, bool MIXED, int W>
+template <typename VT, bool MIXED, int W, bool PACKED>
 __global__ void __launch_bounds__(TFS_TPB, sizeof(VT) == 4 ? TFS_PIPE_MINB32 : TFS_PIPE_MINB64)
 k_spmv_pq_pipe(SellDev A, const VT *__restrict__ val, const VT *__restrict__ p, VT *__restrict__ q,
                DevState *st, double *part)
@@ -98,7 +99,7 @@ k_spmv_pq_pipe(SellDev A, const VT *__restrict__ val, const VT *__restrict__ p, 
         last = grid_reduce_f<1>(a1, v, part, &st->counter);
     } else {
         v[0] = (double)acc;
-        last = grid_reduce<1>(v, part, &st->counter);
+        last = grid_reduce<1, PACKED>(v, part, &st->counter);
     }
     if (last) {
         st->alpha = st->rho / v[0];
