@@ -338,7 +338,8 @@ def run_ours(args, dist: Dist) -> dict | None:
     # level step splits into the hand-off between launches (the wait for the
     # previous level's completion) and the launch's own work.
     level_split = None
-    if prec == 2 and sol.stats()["dic_kernel"] == 0:
+    tiled = prec == 2 and sol.stats()["dic_tiles"] > 0
+    if prec == 2 and not tiled and sol.stats()["dic_kernel"] == 0:
         prof = sol.profile_prec(s.val, TFS_MIXED)
         work = [p["end_us"] - p["start_us"] for p in prof]
         gaps = [b["start_us"] - a["end_us"] for a, b in zip(prof, prof[1:])]
@@ -437,16 +438,18 @@ def run_ours(args, dist: Dist) -> dict | None:
                  "timing": "CUDA events, back-to-back launches on the handle's stream"}
     roof = roof_spmv
     if prec32_ms is not None:
-        # The level sweeps are the dominant kernels of DIC-CG: one "launch" is
-        # one preconditioner application (all level kernels of both sweeps).
+        # The sweeps are the dominant kernels of DIC-CG: one "launch" is one
+        # preconditioner application (both sweeps).
         ach = prec_bytes32 / (prec32_ms * 1e-3) / 1e9
-        roof = {"kernel": "k_sweep_level + k_sweep_tail1 (one binary32 DIC application: "
+        roof = {"kernel": "k_dic_tile<float, 0> + k_dic_tile<float, 1> (one binary32 DIC application: "
+                          "forward and backward sweep, tile by tile)" if tiled else
+                          "k_sweep_level + k_sweep_tail1 (one binary32 DIC application: "
                           "forward levels, fused tails, backward levels)",
                 "bound": "hbm", "achieved": round(ach, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(ach / peak, 4), "peak_source": f"{peak_src} hbm_gbs",
                 "algorithmic_bytes_per_launch": prec_bytes32,
                 "us_per_application": round(prec32_ms * 1e3, 2), "level_split": level_split,
-                "traffic": ncu_traffic(args.workload, "dic_application"),
+                "traffic": ncu_traffic(args.workload, "dic_tiles" if tiled else "dic_application"),
                 "timing": "CUDA events, back-to-back applications on the handle's stream"}
     mixed = results.get("mixed") or results["fp64"]
     fp64 = results.get("fp64") or mixed

@@ -15,12 +15,24 @@
 //     padding) come through a ring in rounds of up to TILE_ROWS rows, one
 //     bulk copy (cp.async.bulk) a round into a place fixed by the plan,
 //     issued by a copy lane as the rounds it overwrites are released;
-//   - a row's right-hand side is gathered from the solver's row order by a
-//     4- or 8-byte cp.async straight into the row's own slot, TILE_PF rounds
-//     ahead, its row word (row, entry count, own or closure) as many rounds
-//     before that;
-//   - every row of the closure is swept, only the tile's own rows are stored;
-//     the forward sweep stores the backward start values y / (D + TINY).
+//   - the vectors move between the solver's row order and the slots by
+//     threads of their own, level by level and in the order of the rows:
+//     loaders bring every row's right-hand side by a 4- or 8-byte cp.async
+//     into its slot, storers (binary32) take the own rows out;
+//   - every row of the closure is swept, only the tile's own rows are stored.
+//     In binary64 the forward sweep stores the backward start values
+//     y / (D + TINY) by tile_quotient; in binary32 it stores y and the
+//     backward sweep divides.
+// An application alone, us, level kernels -> tiles: 128^3 binary32 98 -> 51,
+// binary64 219 -> 141; 64^3 52 -> 19 and 92 -> 39.  In binary64 the pipe
+// bounds it (77 us of the 141 at 128^3 are its instructions alone); in
+// binary32 and on small meshes the chain of a level's gathers, products and
+// barrier does, about 0.5 us a level (128^3: 35% of the DRAM's rate, 45% of
+// the issue slots).  Slower: rounds of 1024 rows, two or three tiles a
+// multiprocessor (57 and 78 us), row words in a register queue moved along
+// every round (each move waits for its load), operands loaded before the
+// barrier (64), a seven-way switch over the widths unrolled four times (it
+// leaves the instruction cache).
 // Every row does exactly sweep_row's operations in sweep_row's order, so the
 // sweeps are bitwise those of the level kernels.
 //
@@ -36,11 +48,8 @@
 namespace tfs {
 
 constexpr int TILE_TPB = TILE_ROWS + 2 * TILE_MOVERS + 32;   // row threads, loaders, storers and a copy warp
-#ifndef TFS_TILE_BATCH
-#define TFS_TILE_BATCH 8
-#endif
 constexpr int TILE_QUIT = 2;                              // abort flag of a sweep that has nothing to do
-constexpr int TILE_BATCH = TFS_TILE_BATCH;                // list rounds whose rows a mover holds at once
+constexpr int TILE_BATCH = 8;                             // list rounds whose rows a mover holds at once
 
 // One direction of a plan on the device.
 struct TileDev {

@@ -33,10 +33,7 @@
 
 namespace tfs {
 
-#ifndef TFS_TILE_ROWS
-#define TFS_TILE_ROWS 512                // rows of a round (a row per thread); a multiple of 32, at most 992
-#endif
-constexpr int TILE_ROWS = TFS_TILE_ROWS;
+constexpr int TILE_ROWS = 512;           // rows of a round (a row per thread); a multiple of 32, at most 992
 constexpr int TILE_SLICES = TILE_ROWS / 32;
 constexpr uint32_t TILE_ROW_MASK = 0x03ffffffu;  // row word: internal row,
 constexpr int TILE_CNT_SHIFT = 26;               // entries on the swept side (0..15) << 26,
@@ -47,10 +44,7 @@ constexpr int TILE_MAX_ROUNDS = 512;     // rounds of one tile and direction
 constexpr int TILE_MAX_SLOTS = 65504;    // slots of one tile: 16-bit entry indices
 constexpr int TILE_MAX_LEVELS = 64;      // deeper schedules have long closures
 constexpr int TILE_BARS = 16;            // rounds staged ahead at most
-#ifndef TFS_TILE_MOVERS
-#define TFS_TILE_MOVERS 224              // threads that move vectors one way: rows of a list round
-#endif
-constexpr int TILE_MOVERS = TFS_TILE_MOVERS;
+constexpr int TILE_MOVERS = 224;         // threads that move vectors one way: rows of a list round
 constexpr int TILE_MAX_LISTS = 1024;     // list rounds of one tile and direction
 constexpr int TILE_HEAD = 128;           // bytes of a round's head: a word per slice
 
@@ -509,15 +503,9 @@ inline TilePlan tile_plan(int n, const std::vector<int> &row0, const std::vector
 // while a tile's rows (about 1.35 times its own) fit beside the ring in
 // binary64, fewer where tiles would drop below about 1500 own rows (their
 // closures would outweigh them).
-#ifndef TFS_TILE_CAP
-#define TFS_TILE_CAP 14400
-#endif
-#ifndef TFS_TILE_LEAST
-#define TFS_TILE_LEAST 1536
-#endif
 inline int tile_count(int n, int sms)
 {
-    const int cap = TFS_TILE_CAP, least = TFS_TILE_LEAST;
+    const int cap = 14400, least = 1536;
     if (n < 2 * least) return 1;
     if ((int64_t)n < (int64_t)least * sms) return n / least;
     return sms * (int)(((int64_t)n + (int64_t)sms * cap - 1) / ((int64_t)sms * cap));

@@ -1009,9 +1009,7 @@ static bool level_options_default(const tfs_handle *h)
 
 // Shared memory of a block's ring at most: what is in flight covers the
 // memory's latency well before this.
-#ifndef TFS_TILE_RING
 #define TFS_TILE_RING (96 << 10)
-#endif
 
 // The tiled DIC's plan for the current layout and arithmetic T, made on the
 // first DIC solve (the topology is fixed, so once per mesh).  A plan that does
