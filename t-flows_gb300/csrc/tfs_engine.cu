@@ -252,12 +252,15 @@ static void launch_spmv_pipe(const tfs_handle *h, cudaStream_t s, const VT *val,
     auto launch_ex = [l1](bool on, auto kernel, int grid, int block, cudaStream_t st, auto... args) {
         return launch_ex_l1(l1, on, kernel, grid, block, st, args...);
     };
-    // (l1: the block sums by shuffles, whose 64 bytes leave the L1 whole;
-    // else packed: a 64^3 binary64 SpMV 17.5 -> 15.9 us after tiled sweeps.)
+    // SMALL: binary64 unless all of the L1 is asked for (its block sums then go
+    // by shuffles, whose 64 bytes leave it whole); binary32 from where the
+    // unconstrained kernel's four blocks an SM do not hold the grid to three
+    // chunks a block of the full grid.
+    const bool small = MIXED ? h->n_chunks > 4 * h->sm_count && h->n_chunks <= 24 * h->sm_count : !l1;
     auto width = [&](auto w) {
         constexpr int W = decltype(w)::value;
-        if (MIXED || l1) launch_ex(pdl, k_spmv_pq_pipe<VT, MIXED, W, false>, G, TFS_TPB, s, A, val, p, q, h->st, h->part);
-        else launch_ex(pdl, k_spmv_pq_pipe<VT, MIXED, W, !MIXED>, G, TFS_TPB, s, A, val, p, q, h->st, h->part);
+        if (small) launch_ex(pdl, k_spmv_pq_pipe<VT, MIXED, W, true>, G, TFS_TPB, s, A, val, p, q, h->st, h->part);
+        else launch_ex(pdl, k_spmv_pq_pipe<VT, MIXED, W, false>, G, TFS_TPB, s, A, val, p, q, h->st, h->part);
     };
     switch (h->sell_width) {
     case 1: width(std::integral_constant<int, 1>{}); break;

@@ -24,8 +24,13 @@ namespace tfs {
 
 // q = A p; (p, q); alpha, software-pipelined over the thread's rows c *
 // 256 + tid, c = blockIdx.x, blockIdx.x + gridDim.x, ... (the direct
-// kernels' rows and order).  W: the matrix's uniform slice width.  PACKED:
-// block_sum_packed (binary64).
+// kernels' rows and order).  W: the matrix's uniform slice width.
+// SMALL: in binary64 the block sums packed (block_sum_packed; 64^3 17.5 -> 15.9
+// us); in binary32 eight blocks an SM, the whole grid in one wave: with a few
+// chunks a block the kernel waits for its first rows' loads, and twice the
+// warps wait at once (64^3 9.9 -> 7.7 us after tiled sweeps, 8.8 -> 7.2 in a
+// diagonal CG, 90^3 13.3 -> 11.4 there), while a long row loop loses more to
+// the spills of 32 registers (128^3 29.4 -> 32.1).
 // Minimum resident blocks per SM asked of the compiler (register cap).
 // Unconstrained (1) is kept: on the 128^3 system the binary32 kernel runs
 // at 52 registers (4 blocks per SM) in 31.5 us; capped to 47 or 40
@@ -39,8 +44,8 @@ namespace tfs {
 #ifndef TFS_PIPE_MINB64
 #define TFS_PIPE_MINB64 1
 #endif
-template <typename VT, bool MIXED, int W, bool PACKED>
-__global__ void __launch_bounds__(TFS_TPB, sizeof(VT) == 4 ? TFS_PIPE_MINB32 : TFS_PIPE_MINB64)
+template <typename VT, bool MIXED, int W, bool SMALL>
+__global__ void __launch_bounds__(TFS_TPB, sizeof(VT) == 4 ? (SMALL ? 8 : TFS_PIPE_MINB32) : TFS_PIPE_MINB64)
 k_spmv_pq_pipe(SellDev A, const VT *__restrict__ val, const VT *__restrict__ p, VT *__restrict__ q,
                DevState *st, double *part)
 {
@@ -99,7 +104,7 @@ k_spmv_pq_pipe(SellDev A, const VT *__restrict__ val, const VT *__restrict__ p, 
         last = grid_reduce_f<1>(a1, v, part, &st->counter);
     } else {
         v[0] = (double)acc;
-        last = grid_reduce<1, PACKED>(v, part, &st->counter);
+        last = grid_reduce<1, SMALL>(v, part, &st->counter);
     }
     if (last) {
         st->alpha = st->rho / v[0];
