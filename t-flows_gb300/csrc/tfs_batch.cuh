@@ -62,15 +62,22 @@ struct BatchCtl {
 
 #define TFS_BATCH_MAX_TPB 512
 // CTAs of 512 threads an SM is to hold: one (128 registers, no spilling) or,
-// for binary32 batches that ask for more CTAs than TFS_BATCH_ROOMY an SM, two
-// (64 registers, 90 bytes spilled).  Measured, one / two, ms: 24 systems of
+// for batches that ask for more CTAs than TFS_BATCH_ROOMY (binary64:
+// TFS_BATCH_CROWDED) an SM, two (64 registers, some spilling).  Measured, one / two, ms: 24 systems of
 // 5k to 91k cells mixed 16 x 512 10.6 / 10.2, 8 x 512 9.6 / 14.0; 96 systems
 // of up to 500k cells mixed 16 x 512 235 / 197, 8 x 512 221 / 215; binary64
 // 24 systems 27.7 / 31.7 and 39.9 / 43.6, 96 systems 608 / 583 and 539 / 569.
 // (Three, as long as the whole system's pointers and every thread's copy of
 // the solve's scalars were spilled: 20.8 and 21.5, 249 and 353; binary64 45.8
 // and 48.7, 622 and 751.)
+// Binary64 by CTAs asked for per SM, one / two / three, ms: 3.4 (64 systems of
+// up to 500k cells, 8 x 512) 366 / 490 / 655, 6.7 (16 x 512) 337 / 341 / 478,
+// 13.5 (256 systems, 8 x 512) 1267 / 1043 / 1127, 27 (16 x 512) 1439 / 1375 /
+// 1418.  Binary32 with DIC, whose level barriers leave most to wait for, two /
+// three: 5.1 (96 systems, 8 x 512, 60 iterations) 87 / 105, 8.4 (160 systems)
+// 132 / 120.
 #define TFS_BATCH_ROOMY 3
+#define TFS_BATCH_CROWDED 8
 
 // Sum of NV values over the cluster: block sum, one partial per CTA in
 // shared memory, cluster barrier, the C partials added in rank order.  The

@@ -2398,9 +2398,11 @@ extern "C" int tfs_batch_configure(tfs_batch *b, int cluster_size, int threads_p
 template <int METHOD, typename VT>
 static int launch_batch_kernel(tfs_batch *b)
 {
-    auto kernel = k_batch<METHOD, VT, 1>;
-    if constexpr (sizeof(VT) == 4)
-        if ((int64_t)b->n * b->cluster > (int64_t)TFS_BATCH_ROOMY * b->hs[0]->sm_count) kernel = k_batch<METHOD, VT, 2>;
+    const int64_t asked = (int64_t)b->n * b->cluster, sms = b->hs[0]->sm_count;
+    auto kernel = asked > (sizeof(VT) == 4 ? TFS_BATCH_ROOMY : TFS_BATCH_CROWDED) * sms ? k_batch<METHOD, VT, 2>
+                                                                                        : k_batch<METHOD, VT, 1>;
+    if constexpr (METHOD == 2 && sizeof(VT) == 4)
+        if (asked > TFS_BATCH_CROWDED * sms) kernel = k_batch<METHOD, VT, 3>;
     if (b->cluster > 8) CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];

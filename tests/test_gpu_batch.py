@@ -149,21 +149,22 @@ def test_batch_literal_bicg_refuses_dic(systems):
                 b.solve(TFS_BICG, 2, [s.val], [np.zeros(s.n)], [s.b.copy()], 100, [1e-8])
 
 
-def test_batch_crowded_equals_alone(gpu):
-    """A mixed batch that asks for more CTAs than three an SM runs the kernel
-    compiled for two of them per SM, a smaller batch the one compiled for one:
-    the same bits."""
-    systems = [system(POISSON, 5 + k % 4, 6, 7, seed=100 + k) for k in range(36)]
-    sols = [Solver(s.matrix(), precision=TFS_MIXED) for s in systems]
+@pytest.mark.parametrize("mode,count", [(TFS_MIXED, 36), (TFS_MIXED, 80), (TFS_FP64, 80)])
+def test_batch_crowded_equals_alone(mode, count, gpu):
+    """A batch that asks for more CTAs than three (binary64: eight) an SM runs
+    the kernel compiled for two of them per SM (mixed DIC past eight: three), a
+    smaller batch the one compiled for one: the same bits."""
+    systems = [system(POISSON, 5 + k % 4, 6, 7, seed=100 + k) for k in range(count)]
+    sols = [Solver(s.matrix(), precision=mode) for s in systems]
     tols = [1e-8 * float(np.linalg.norm(s.b)) for s in systems]
     for prec in (1, 2):
         xs, rs = [np.zeros(s.n) for s in systems], [s.b.copy() for s in systems]
         with Batch(sols, 16, 512) as b:
-            res = b.solve(TFS_CG, prec, [s.val for s in systems], xs, rs, 500, tols, mode=TFS_MIXED)
-        for k in (0, 17, 35):
+            res = b.solve(TFS_CG, prec, [s.val for s in systems], xs, rs, 500, tols, mode=mode)
+        for k in (0, 17, count - 1):
             x, r = [np.zeros(systems[k].n)], [systems[k].b.copy()]
             with Batch([sols[k]], 16, 512) as b:
-                one = b.solve(TFS_CG, prec, [systems[k].val], x, r, 500, [tols[k]], mode=TFS_MIXED)
+                one = b.solve(TFS_CG, prec, [systems[k].val], x, r, 500, [tols[k]], mode=mode)
             assert one.niter[0] == res.niter[k] and np.array_equal(x[0], xs[k]) and np.array_equal(r[0], rs[k])
     for s in sols:
         s.close()
