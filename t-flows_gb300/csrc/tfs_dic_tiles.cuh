@@ -39,7 +39,8 @@
 // Every wait is on the block's own copies or its own warps, and bounded as in
 // the one-block DIC: a wait that runs out raises the block's abort flag,
 // after which no copy is issued and no slot is read, and the solve ends with
-// TFS_ERR_TIMEOUT.
+// TFS_ERR_TIMEOUT.  The copy lane stays until what it issued has landed,
+// whether the sweep was finished, called off or never begun (tile_copy_walk).
 #pragma once
 #include "tfs_dic_block.cuh"
 #include "tfs_dic_tiles_plan.h"
@@ -172,6 +173,41 @@ __device__ __forceinline__ bool tile_wait(uint64_t *bar, unsigned parity, volati
     return dicb_mbar_test(bar, parity) || tile_wait_slow(bar, parity, abort, wait_ns);
 }
 
+// What the copy lane does for a round (tile_copy_walk).
+struct TileCopy {
+    const uint4 *tab;
+    unsigned char *ring;
+    const unsigned char *packed;
+    uint64_t *full, *empty;
+    volatile int *abort;
+    unsigned long long wait_ns;
+    uint4 c;                            // the round that back() looked at last
+    __device__ int back(int k)
+    {
+        c = tab[k];
+        return (int)(c.y >> 16 & 0xffu);
+    }
+    __device__ bool released(int k)
+    {
+        return tile_wait_empty(empty + k % TILE_BARS, (unsigned)(k / TILE_BARS) & 1u, abort, wait_ns);
+    }
+    __device__ bool off() { return *abort != 0; }
+    __device__ void issue(int k)
+    {
+        uint64_t *bar = full + k % TILE_BARS;
+        const unsigned bytes = (c.y & 0xffffu) * 16u;
+        dicb_mbar_expect(bar, bytes);
+        dicb_bulk(ring + (c.w & 0xffffu) * 128u, packed + 16 * (size_t)c.x, bytes, bar);
+    }
+    // (bounded as every wait, but the flag is not asked)
+    __device__ void landed(int k)
+    {
+        const unsigned long long t0 = gtimer();
+        while (!dicb_mbar_test(full + k % TILE_BARS, (unsigned)(k / TILE_BARS) & 1u) && gtimer() - t0 < wait_ns) {
+        }
+    }
+};
+
 // The vectors between global memory and the tile's slots, by two sets of
 // TILE_MOVERS threads (m: this one's number in its set), level by level: the
 // loaders every row's right-hand side, asynchronously; the storers the own
@@ -280,22 +316,8 @@ k_dic_tile(TileDev P, const T *__restrict__ src, T *__restrict__ dst, DevState *
             tile_prefetch(P.list_row + (size_t)l0 * TILE_MOVERS, (unsigned)n * TILE_MOVERS * 4u);
             tile_prefetch(P.list_slot + (size_t)l0 * TILE_MOVERS, (unsigned)n * TILE_MOVERS * 2u);
         }
-        int k = 0;
-        for (; k < rounds && !*abort; k++) {
-            const uint4 c = tab[k];
-            const int back = (int)(c.y >> 16 & 0xffu), dep = k - back;
-            if (back && !tile_wait_empty(empty + dep % TILE_BARS, (unsigned)(dep / TILE_BARS) & 1u, abort, wait_ns)) break;
-            uint64_t *bar = full + k % TILE_BARS;
-            const unsigned bytes = (c.y & 0xffffu) * 16u;
-            dicb_mbar_expect(bar, bytes);
-            dicb_bulk(ring + (c.w & 0xffffu) * 128u, P.packed + 16 * (size_t)c.x, bytes, bar);
-        }
-        // after an abort, wait (bounded) for the copies still in flight
-        for (int q = k > TILE_BARS ? k - TILE_BARS : 0; q < k && *abort; q++) {
-            const unsigned long long t0 = gtimer();
-            while (!dicb_mbar_test(full + q % TILE_BARS, (unsigned)(q / TILE_BARS) & 1u) && gtimer() - t0 < wait_ns) {
-            }
-        }
+        TileCopy copy{tab, ring, P.packed, full, empty, abort, wait_ns, make_uint4(0u, 0u, 0u, 0u)};
+        tile_copy_walk(rounds, copy);
         return;
     }
     const int warp = tid >> 5, lane = tid & 31;
@@ -303,7 +325,7 @@ k_dic_tile(TileDev P, const T *__restrict__ src, T *__restrict__ dst, DevState *
     cudaGridDependencySynchronize();
     const unsigned long long diag = st->dicb_wait_ns;
     const unsigned long long wait_ns = diag ? diag : TFS_DICB_WAIT_NS;
-    if (st->done) {   // nothing to sweep: the copy lane leaves as after an abort
+    if (st->done) {   // nothing to sweep: the copy lane issues no more
         if (tid == 0) *abort = TILE_QUIT;
         return;
     }

@@ -137,6 +137,34 @@ inline bool tile_place(TileRound *r, int n, int ring)
     return true;
 }
 
+// The copy lane's walk over a tile's rounds: the kernel's, and on the host its
+// test's.  C: back(k) how many rounds back the last one is that round k
+// overwrites (0: none); released(k) waits until the row warps have released
+// round k, false when that wait ends otherwise; off() whether the sweep has
+// been called off; issue(k) starts round k's copy; landed(k) waits for it.
+//   - The flag is asked after the wait: in a sweep that is called off, rounds
+//     are released that have not landed.
+//   - The last rounds issued are waited for however the walk ends.  Those
+//     before them have landed, since one of these overwrites them.  Asking the
+//     flag whether to wait is not enough: a sweep that has nothing to do is
+//     called off after its dependency wait, when the lane of a tile whose
+//     rounds all fit the ring is long through, and the block would leave with
+//     copies on their way into shared memory that is another's by then.
+template <class C>
+#ifdef __CUDACC__
+__device__
+#endif
+inline void tile_copy_walk(int rounds, C &c)
+{
+    int k = 0;
+    for (; k < rounds; k++) {
+        const int back = c.back(k);
+        if ((back && !c.released(k - back)) || c.off()) break;
+        c.issue(k);
+    }
+    for (int q = k > TILE_BARS ? k - TILE_BARS : 0; q < k; q++) c.landed(q);
+}
+
 // Runs fn(k) for k in [0, n) on up to `threads` host threads.
 template <class F>
 inline void tile_parallel(int n, int threads, F fn)
