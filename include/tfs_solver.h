@@ -200,6 +200,11 @@ int tfs_get_option(const tfs_handle *h, int option, int *value);
  * Replaces nothing in the reference. */
 int tfs_diag_dic_timeout(tfs_handle *h, long long wait_ns);
 
+/* Diagnostics of the paths that do without device memory: the nth device
+ * allocation of the handle from now on (1: the next one; 0: none) fails as if
+ * the device had no more.  Replaces nothing in the reference. */
+int tfs_diag_alloc_failure(tfs_handle *h, int nth);
+
 /* ---- solves ------------------------------------------------------------- */
 
 /* One preconditioned Krylov solve with host arrays (val, x, r1 host memory).

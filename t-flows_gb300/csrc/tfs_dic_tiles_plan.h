@@ -27,6 +27,8 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <exception>
+#include <mutex>
 #include <thread>
 #include <utility>
 #include <vector>
@@ -93,6 +95,18 @@ struct TilePlan {
     int smem_bytes = 0;                  // dynamic shared memory of a sweep
     double redundancy = 0.0;             // rows swept per row, the larger direction
     TileDir dir[2];                      // forward, backward
+
+    // Device bytes of its arrays.
+    int64_t bytes() const
+    {
+        int64_t b = 0;
+        for (const TileDir &D : dir)
+            b += (int64_t)(4 * (D.tile_round.size() + D.tile_list.size() + D.rows.size() + D.vbeg.size() +
+                                D.list_row.size()) +
+                           2 * D.list_slot.size() + D.packed.size() + D.lists.size() +
+                           sizeof(TileRound) * D.rounds.size());
+        return b;
+    }
 };
 
 // Dynamic shared memory of a sweep: the tile's vector, the ring, the round
@@ -165,19 +179,34 @@ inline void tile_copy_walk(int rounds, C &c)
     for (int q = k > TILE_BARS ? k - TILE_BARS : 0; q < k; q++) c.landed(q);
 }
 
-// Runs fn(k) for k in [0, n) on up to `threads` host threads.
+// Runs fn(k, thread) for k in [0, n) on up to `threads` host threads, fewer
+// where the system refuses to start one.  An exception of fn ends the run and
+// is thrown again here, once every thread is through.
 template <class F>
 inline void tile_parallel(int n, int threads, F fn)
 {
     threads = std::max(1, std::min(threads, n));
     std::atomic<int> next{0};
+    std::exception_ptr error;
+    std::mutex mu;
     auto work = [&](int t) {
-        for (int k; (k = next.fetch_add(1)) < n;) fn(k, t);
+        try {
+            for (int k; (k = next.fetch_add(1)) < n;) fn(k, t);
+        } catch (...) {
+            next = n;
+            std::lock_guard<std::mutex> lock(mu);
+            if (!error) error = std::current_exception();
+        }
     };
     std::vector<std::thread> pool;
-    for (int t = 1; t < threads; t++) pool.emplace_back(work, t);
+    pool.reserve((size_t)threads);
+    try {
+        for (int t = 1; t < threads; t++) pool.emplace_back(work, t);
+    } catch (const std::exception &) {   // the threads there are do the work
+    }
     work(0);
     for (auto &t : pool) t.join();
+    if (error) std::rethrow_exception(error);
 }
 
 // Rows (in the order `pos`, which keeps mesh neighbours close) into `tiles`
@@ -281,6 +310,7 @@ inline void tile_partition(int n, const std::vector<int> &adj_ptr, const std::ve
 // and the internal row of every row.  tiles: how many; max_ratio: the most
 // rows swept per row, beyond which there is no plan; ts: bytes of a value;
 // optin: shared memory a block can have, ring_most: of it for the ring.
+// Throws std::bad_alloc where the host has no memory for it.
 inline TilePlan tile_plan(int n, const std::vector<int> &row0, const std::vector<int> &col0,
                           const std::vector<int> &dia0, const std::vector<int32_t> &level,
                           const std::vector<int> &pos, const std::vector<int> &internal, int tiles,

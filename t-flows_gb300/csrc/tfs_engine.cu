@@ -32,7 +32,7 @@ using namespace tfs;
 
 // The tiled DIC's plan (tfs_dic_tiles_plan.h) of one arithmetic on the device.
 struct TileStore {
-    int tiles = 0;                       // 0: no plan, the level kernels sweep
+    int tiles = 0;                       // 0: no plan to be had, the level kernels sweep
     int max_slots = 0, max_rounds = 0, max_lists = 0, ring_bytes = 0, smem_bytes = 0;
     struct Dir {
         TileRound *rounds = nullptr;
@@ -219,7 +219,13 @@ static int dalloc(tfs_handle *h, T **p, size_t count)
 {
     size_t bytes = count * sizeof(T);
     if (bytes == 0) bytes = sizeof(T);
-    CK(cudaMalloc((void **)p, bytes));
+    cudaError_t e = cudaMalloc((void **)p, bytes);
+    if (e == cudaSuccess && h->diag_alloc > 0 && --h->diag_alloc == 0) {   // tfs_diag_alloc_failure
+        cudaFree(*p);
+        *p = nullptr;
+        e = cudaErrorMemoryAllocation;
+    }
+    if (e != cudaSuccess) return tfs_engine_error(e, "cudaMalloc");
     h->device_bytes += (int64_t)bytes;
     return TFS_OK;
 }
@@ -540,14 +546,22 @@ static void rcm_order(int n, const std::vector<int> &row0, const std::vector<int
     for (int k = 0; k < n; k++) rcm_pos[order[k]] = k;
 }
 
+static void free_tiles(TileStore &S)
+{
+    for (TileStore::Dir &D : S.dir) {
+        for (void *p : {(void *)D.rounds, (void *)D.tile_round, (void *)D.vbeg, (void *)D.rows, (void *)D.packed,
+                        (void *)D.tile_list, (void *)D.lists, (void *)D.list_row, (void *)D.list_slot})
+            if (p) cudaFree(p);
+        D = TileStore::Dir{};
+    }
+    S.tiles = 0;
+}
+
 static void free_tiles(tfs_handle *h)
 {
     for (TileStore *&S : h->tiles) {
         if (!S) continue;
-        for (TileStore::Dir &D : S->dir)
-            for (void *p : {(void *)D.rounds, (void *)D.tile_round, (void *)D.vbeg, (void *)D.rows, (void *)D.packed,
-                            (void *)D.tile_list, (void *)D.lists, (void *)D.list_row, (void *)D.list_slot})
-                if (p) cudaFree(p);
+        free_tiles(*S);
         delete S;
         S = nullptr;
     }
@@ -940,6 +954,16 @@ extern "C" int tfs_diag_dic_timeout(tfs_handle *h, long long wait_ns)
     return TFS_OK;
 }
 
+extern "C" int tfs_diag_alloc_failure(tfs_handle *h, int nth)
+{
+    if (!h || nth < 0) {
+        tfs_set_error_text("tfs_diag_alloc_failure: null handle or negative number");
+        return TFS_ERR_ARG;
+    }
+    h->diag_alloc = nth;
+    return TFS_OK;
+}
+
 extern "C" int tfs_get_option(const tfs_handle *h, int option, int *value)
 {
     if (!h || !value) return TFS_ERR_ARG;
@@ -1014,61 +1038,93 @@ static bool level_options_default(const tfs_handle *h)
 // memory's latency well before this.
 #define TFS_TILE_RING (96 << 10)
 
-// The tiled DIC's plan for the current layout and arithmetic T, made on the
-// first DIC solve (the topology is fixed, so once per mesh).  A plan that does
-// not exist, or does not fit the room a server left, leaves tiles = 0: the
+// The tiled DIC's plan for the current layout in values of T; tiles = 0 where
+// there is none, or the host has no memory for making it.
+template <typename T>
+static TilePlan make_tiles(const tfs_handle *h, int optin)
+{
+    TilePlan P;
+    try {
+        const int threads = std::max(1, std::min(16, (int)std::thread::hardware_concurrency()));
+        std::vector<int> internal(h->n);
+        for (int k = 0; k < h->n_int; k++)
+            if (h->perm_host[k] >= 0) internal[h->perm_host[k]] = k;
+        for (int tries = 0, tiles = tile_count(h->n, h->sm_count); tries < 2 && !P.tiles; tries++, tiles += h->sm_count)
+            P = tile_plan(h->n, h->row0, h->col0, h->dia0, h->levels_nat, h->rcm_pos, internal, tiles,
+                          TFS_TILE_MAX_RATIO, sizeof(T), optin, TFS_TILE_RING, threads);
+    } catch (const std::exception &) {
+        P.tiles = 0;
+    }
+    return P;
+}
+
+// Copies a plan to the device.  Device memory that is not to be had is no
+// error: what was taken is given back, and the level kernels, which need none
+// of it, sweep.
+static int upload_tiles(tfs_handle *h, TileStore &S, const TilePlan &P)
+{
+    cudaStream_t s = h->stream;
+    const int64_t before = h->device_bytes;
+    bool full = false;
+    int rc = TFS_OK;
+    auto up = [&](auto **dst, const auto &src) {
+        if (rc || full) return;
+        if (dalloc(h, dst, src.size())) {
+            full = true;
+            cudaGetLastError();
+            return;
+        }
+        const cudaError_t e = cudaMemcpyAsync(*dst, src.data(), sizeof(src[0]) * src.size(), cudaMemcpyHostToDevice, s);
+        if (e != cudaSuccess) rc = tfs_engine_error(e, "tile plan upload");
+    };
+    for (int d = 0; d < 2; d++) {
+        const TileDir &D = P.dir[d];
+        TileStore::Dir &E = S.dir[d];
+        E.n_rounds = (int)D.rounds.size();
+        up(&E.rounds, D.rounds);
+        up(&E.tile_round, D.tile_round);
+        up(&E.vbeg, D.vbeg);
+        up(&E.rows, D.rows);
+        up(&E.packed, D.packed);
+        up(&E.tile_list, D.tile_list);
+        up(&E.lists, D.lists);
+        up(&E.list_row, D.list_row);
+        up(&E.list_slot, D.list_slot);
+    }
+    const cudaError_t e = cudaStreamSynchronize(s);   // the copies read P
+    if (!rc && e != cudaSuccess) rc = tfs_engine_error(e, "tile plan upload");
+    if (rc || full) {
+        free_tiles(S);
+        h->device_bytes = before;
+        return rc;
+    }
+    S.max_slots = P.max_slots;
+    S.max_rounds = P.max_rounds;
+    S.max_lists = P.max_lists;
+    S.ring_bytes = P.ring_bytes;
+    S.smem_bytes = P.smem_bytes;
+    S.tiles = P.tiles;
+    h->stats.device_bytes = h->device_bytes;
+    return TFS_OK;
+}
+
+// The plan of arithmetic T, made on the first DIC solve (the topology is
+// fixed, so once per mesh).  A plan that does not exist, does not fit the room
+// a server left or cannot be had for want of memory leaves tiles = 0: the
 // level kernels sweep.
 template <typename T>
 static int ensure_tiles(tfs_handle *h)
 {
     TileStore *&S = h->tiles[sizeof(T) == 8];
     if (!h->dic_tiles || h->layout != TFS_LAYOUT_LEVELS || !level_options_default(h) || S) return TFS_OK;
-    S = new TileStore;
     int optin = 0;
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
-    const int threads = std::max(1, std::min(16, (int)std::thread::hardware_concurrency()));
-    std::vector<int> internal(h->n);
-    for (int k = 0; k < h->n_int; k++)
-        if (h->perm_host[k] >= 0) internal[h->perm_host[k]] = k;
-    TilePlan P;
-    for (int tries = 0, tiles = tile_count(h->n, h->sm_count); tries < 2 && !P.tiles; tries++, tiles += h->sm_count)
-        P = tile_plan(h->n, h->row0, h->col0, h->dia0, h->levels_nat, h->rcm_pos, internal, tiles, TFS_TILE_MAX_RATIO,
-                      sizeof(T), optin, TFS_TILE_RING, threads);
-    if (!P.tiles) return TFS_OK;
-    int64_t bytes = 0;
-    for (TileDir &D : P.dir)
-        bytes += (int64_t)(D.rows.size() * 8 + D.packed.size() + D.rounds.size() * sizeof(TileRound) +
-                           D.list_row.size() * 6 + D.lists.size());
-    if (bytes > h->tile_room) return TFS_OK;
-    cudaStream_t s = h->stream;
-    int rc;
-    for (int d = 0; d < 2; d++) {
-        TileDir &D = P.dir[d];
-        TileStore::Dir &E = S->dir[d];
-        E.n_rounds = (int)D.rounds.size();
-        auto up = [&](auto **dst, const auto &src) -> int {
-            if (int rc = dalloc(h, dst, src.size())) return rc;
-            CK(cudaMemcpyAsync(*dst, src.data(), sizeof(src[0]) * src.size(), cudaMemcpyHostToDevice, s));
-            return TFS_OK;
-        };
-        if ((rc = up(&E.rounds, D.rounds)) || (rc = up(&E.tile_round, D.tile_round)) || (rc = up(&E.vbeg, D.vbeg)) ||
-            (rc = up(&E.rows, D.rows)) || (rc = up(&E.packed, D.packed)) || (rc = up(&E.tile_list, D.tile_list)) ||
-            (rc = up(&E.lists, D.lists)) || (rc = up(&E.list_row, D.list_row)) || (rc = up(&E.list_slot, D.list_slot))) {
-            cudaStreamSynchronize(s);
-            return rc;
-        }
-    }
-    CK(cudaStreamSynchronize(s));
     CK(cudaFuncSetAttribute(k_dic_tile<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     CK(cudaFuncSetAttribute(k_dic_tile<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-    S->max_slots = P.max_slots;
-    S->max_rounds = P.max_rounds;
-    S->max_lists = P.max_lists;
-    S->ring_bytes = P.ring_bytes;
-    S->smem_bytes = P.smem_bytes;
-    S->tiles = P.tiles;
-    h->stats.device_bytes = h->device_bytes;
-    return TFS_OK;
+    const TilePlan P = make_tiles<T>(h, optin);
+    S = new TileStore;
+    if (!P.tiles || P.bytes() > h->tile_room) return TFS_OK;
+    return upload_tiles(h, *S, P);
 }
 
 // Whether the sweeps of arithmetic T run tile by tile: a plan exists, and the

@@ -146,6 +146,7 @@ struct tfs_handle {
     int64_t tile_room = INT64_MAX;     // device bytes the plan may take (a server's budget)
     int tiles_used = 0;                // tiles of the last DIC application launched (0: none)
     unsigned long long dicb_diag_ns = 0;   // tfs_diag_dic_timeout
+    int diag_alloc = 0;                // tfs_diag_alloc_failure: the allocation that fails, counted down
     int l2_window = 1;                 // TFS_OPT_L2_WINDOW: 1 the column indices persisting in L2
     int dicb_used = 0;                 // the last DIC application launched was the one-block kernel
     // One-block DIC per arithmetic: shared memory (0: does not fit), ring
