@@ -239,12 +239,13 @@ static void spmv_kind_setup(tfs_handle *h)
                                                                                 : TFS_SPMV_DIRECT;
 }
 
-// Rows from which the SpMV after tiled sweeps asks for all of the L1 (see
-// launch_spmv_pipe).
+// Rows from which the SpMV after tiled sweeps (tiled) asks for all of the L1
+// (see launch_spmv_pipe).
 #define TFS_SPMV_L1_ROWS (1 << 20)
 
 template <typename VT, bool MIXED>
-static void launch_spmv_pipe(const tfs_handle *h, cudaStream_t s, const VT *val, const VT *p, VT *q, bool pdl)
+static void launch_spmv_pipe(const tfs_handle *h, cudaStream_t s, const VT *val, const VT *p, VT *q, bool pdl,
+                             bool tiled)
 {
     const SellDev A = sell_of(h);
     const int G = h->grid_spmv;
@@ -254,7 +255,7 @@ static void launch_spmv_pipe(const tfs_handle *h, cudaStream_t s, const VT *val,
     // 128^3 system, binary32 34.3 -> 30.0).  A small one would wait longer for
     // the multiprocessors to change over than it gains (64^3 DIC-CG iteration
     // 52.8 us without, 56.3 with; 1,320 cells 40.6 and 41.5).
-    const bool l1 = h->tiles_used && h->n_int >= TFS_SPMV_L1_ROWS;
+    const bool l1 = tiled && h->n_int >= TFS_SPMV_L1_ROWS;
     auto launch_ex = [l1](bool on, auto kernel, int grid, int block, cudaStream_t st, auto... args) {
         return launch_ex_l1(l1, on, kernel, grid, block, st, args...);
     };
@@ -282,14 +283,14 @@ static void launch_spmv_pipe(const tfs_handle *h, cudaStream_t s, const VT *val,
 
 // q = A p, (p, q) and alpha of a CG iteration on stream s, binary32 (mixed)
 // or binary64, with the handle's SpMV kernel over grid_spmv (virtual)
-// blocks.
-static void launch_spmv_pq(tfs_handle *h, cudaStream_t s, bool mixed, bool pdl = false)
+// blocks.  tiled: tiled sweeps precede it in the iteration.
+static void launch_spmv_pq(tfs_handle *h, cudaStream_t s, bool mixed, bool pdl = false, bool tiled = false)
 {
     const SellDev A = sell_of(h);
     const int VG = h->grid_spmv;
     if (h->spmv_kind == TFS_SPMV_PIPE) {
-        if (mixed) launch_spmv_pipe<float, true>(h, s, h->val32, h->f.p, h->f.q, pdl);
-        else launch_spmv_pipe<double, false>(h, s, h->val, h->v.p, h->v.q, pdl);
+        if (mixed) launch_spmv_pipe<float, true>(h, s, h->val32, h->f.p, h->f.q, pdl, tiled);
+        else launch_spmv_pipe<double, false>(h, s, h->val, h->v.p, h->v.q, pdl, tiled);
     } else if (mixed) {
         k_mx_spmv_pq<<<VG, TFS_TPB, 0, s>>>(A, h->val32, h->f.p, h->f.q, h->st, h->part);
     } else {
@@ -1380,7 +1381,7 @@ static int tfs_mixed_body(tfs_handle *h, cudaStream_t s, int method, int prec,
             if ((rc = launch_sweeps<float>(h, s, 1, F.r, nullptr, F.y, nullptr, F.z, nullptr, count))) return rc;
             k_mx_dot_rho<0><<<G, T, 0, s>>>(nc, F, h->st, h->part);
             k_mx_cg_p<true><<<G, T, 0, s>>>(nc, F, h->st);
-            launch_spmv_pq(h, s, true);
+            launch_spmv_pq(h, s, true, false, use_tiles<float>(h));
             k_mx_cg_update<false><<<G, T, 0, s>>>(nc, V, F, h->st, h->part);
             k_mx_fold<<<G, T, 0, s>>>(nc, V, F, h->st);
             k_mx_true<0, false><<<G, T, 0, s>>>(A, h->val, V, F, h->st, h->part, prec, cond);
@@ -1399,7 +1400,7 @@ static int tfs_mixed_body(tfs_handle *h, cudaStream_t s, int method, int prec,
             const bool pv = h->use_pdl && h->pdl_vec;
             if ((rc = launch_sweeps<float>(h, s, 1, F.r, nullptr, F.y, nullptr, F.z, nullptr, count, true))) return rc;
             launch_ex(pv, k_mx_cg_p4, G4, T, s, n4, F, (const DevState *)h->st);
-            launch_spmv_pq(h, s, true, pv);
+            launch_spmv_pq(h, s, true, pv, use_tiles<float>(h));
             launch_ex(pv, k_mx_cg_update4<false>, G4, T, s, n4, F, h->st, h->part, l0 / 4);
             launch_ex(pv, k_mx_fold4, G4, T, s, n4, V, F, (const DevState *)h->st);
             launch_ex(pv, k_mx_true<0, false>, G, T, s, A, (const double *)h->val, V, F, h->st, h->part, prec, cond, l0);
@@ -1411,7 +1412,7 @@ static int tfs_mixed_body(tfs_handle *h, cudaStream_t s, int method, int prec,
             if ((rc = launch_sweeps<float>(h, s, 1, F.r, nullptr, F.y, nullptr, F.z, nullptr, count))) return rc;
             launch_ex(pv, k_mx_dot_rho4, G4, T, s, n4, F, h->st, h->part);
             launch_ex(pv, k_mx_cg_p4, G4, T, s, n4, F, (const DevState *)h->st);
-            launch_spmv_pq(h, s, true, pv);
+            launch_spmv_pq(h, s, true, pv, use_tiles<float>(h));
             launch_ex(pv, k_mx_cg_update4<false>, G4, T, s, n4, F, h->st, h->part, 0);
             launch_ex(pv, k_mx_fold4, G4, T, s, n4, V, F, (const DevState *)h->st);
             launch_ex(pv, k_mx_true<0, false>, G, T, s, A, (const double *)h->val, V, F, h->st, h->part, prec, cond, 0);
@@ -1501,7 +1502,7 @@ static int launch_body(tfs_handle *h, cudaStream_t s, int method, int prec,
             const bool pv = h->use_pdl && h->pdl_vec;   // vector kernels PDL-chained
             if ((rc = launch_sweeps<double>(h, s, 1, V.r, nullptr, V.y, nullptr, V.z, nullptr, count, true))) return rc;
             launch_ex(pv, TFS_STEPS(k_cg_p, true), G, T, s, nc, V, (const DevState *)h->st);
-            launch_spmv_pq(h, s, false, pv);
+            launch_spmv_pq(h, s, false, pv, use_tiles<double>(h));
             launch_ex(pv, TFS_STEPS(k_cg_update, false), G, T, s, nc, V, h->st, h->part, cond, l0);
             *count += 3;
         } else if (prec == 2) {
@@ -1509,7 +1510,7 @@ static int launch_body(tfs_handle *h, cudaStream_t s, int method, int prec,
             if ((rc = launch_sweeps<double>(h, s, 1, V.r, nullptr, V.y, nullptr, V.z, nullptr, count))) return rc;
             launch_ex(pv, TFS_STEPS(k_dot_rho, 0), G, T, s, nc, V, h->st, h->part);
             launch_ex(pv, TFS_STEPS(k_cg_p, true), G, T, s, nc, V, (const DevState *)h->st);
-            launch_spmv_pq(h, s, false, pv);
+            launch_spmv_pq(h, s, false, pv, use_tiles<double>(h));
             launch_ex(pv, TFS_STEPS(k_cg_update, false), G, T, s, nc, V, h->st, h->part, cond, 0);
             *count += 4;
         } else {
@@ -1690,6 +1691,8 @@ static int build_graph(tfs_handle *h, int method, int prec, GraphEntry &ge)
             else rc = launch_body(h, h->stream2, method, prec, cond, &ge.body_kernels);
         }
         if (rc) { fail(cudaErrorUnknown, "body"); return rc; }
+        ge.dic_kernel = h->dicb_used;
+        ge.dic_tiles = h->tiles_used;
         cudaGraph_t btmp;
         e = cudaStreamEndCapture(h->stream2, &btmp);
         if (e != cudaSuccess) return fail(e, "end body capture");
@@ -1815,6 +1818,10 @@ int tfs_solve_launch(int method, tfs_handle *h, const double *val, double *x, do
         if ((rc = run_eager(h, kmethod, prec, ge))) return rc;
     } else {
         CK(cudaGraphLaunch(ge->exec, s));
+        if (prec == 2) {
+            h->dicb_used = ge->dic_kernel;
+            h->tiles_used = ge->dic_tiles;
+        }
     }
     CK(cudaEventRecord(h->ev1, s));
     if (!device_ptrs) {

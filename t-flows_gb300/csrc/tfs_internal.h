@@ -108,6 +108,7 @@ struct GraphEntry {
     cudaGraphExec_t exec = nullptr;
     cudaGraph_t graph = nullptr;
     int prologue_kernels = 0, body_kernels = 0, epilogue_kernels = 0;
+    int dic_kernel = 0, dic_tiles = 0;   // of its sweeps: tfs_handle::dicb_used, tiles_used
 };
 
 struct tfs_handle {
