@@ -200,6 +200,16 @@ int tfs_get_option(const tfs_handle *h, int option, int *value);
  * Replaces nothing in the reference. */
 int tfs_diag_dic_timeout(tfs_handle *h, long long wait_ns);
 
+/* Diagnostics of the binary64 CG that solves a small system in one kernel
+ * (its blocks wait for one another, `looks` times at most, each about a
+ * microsecond).  what 1: one block does not answer the roll call, which is
+ * given up, and the launched kernels solve, to the same bits; what 2: one
+ * block withholds a partial sum, the others' waits run out, and the solve
+ * returns TFS_ERR_TIMEOUT with the GPU unaffected; what 0 with looks 0
+ * restores the normal run.  Holds for the handle's solves that follow.
+ * Replaces nothing in the reference. */
+int tfs_diag_resident(tfs_handle *h, int what, int looks);
+
 /* Diagnostics of the paths that do without device memory: the nth device
  * allocation of the handle from now on (1: the next one; 0: none) fails as if
  * the device had no more.  Replaces nothing in the reference. */

@@ -13,6 +13,15 @@
 // 32^3 17.4 -> 10.3, 38,912 rows (a block per multiprocessor) 18.0 -> 10.6,
 // 77,658 rows (two, the most that are resident) 23.7 -> 19.5.
 //
+// The blocks start with a roll call.  That they are all resident is what a
+// cooperative launch promises; how long it takes beside other work -- a batch,
+// another handle, kernels of the caller's -- is not said anywhere.  A call not
+// answered in full in some 10 ms is given up by all of them; nothing has been
+// touched, nothing is stored, and the host launches the per-iteration kernels
+// instead, which give the same bits.  After the call every block runs, and a
+// wait that runs out is an error.  (The loop in the same graph, for the device
+// to fall back on, would cost every solve the 10 us of a conditional node.)
+//
 // Bitwise the same as those kernels: the same row sums, the block sums and
 // the sum over the blocks' partials in the same order.  A block forms p of a
 // gathered row itself, z + beta p_old (the two operations of k_cg_p), which
@@ -29,9 +38,34 @@ struct alignas(16) CgSlot {
     unsigned long long seq;
 };
 
-// Limit of a wait for the other blocks (all resident and at most a row's
-// work apart).
-#define CG_RESIDENT_WAIT_NS 2000000000ull
+// Looks, of about a microsecond, that a wait for the other blocks takes at
+// most: in the roll call, and in an exchange, whose blocks all run and are at
+// most a row's work apart.  (Looks, not time: a context that is switched off
+// the GPU does not look.)
+#define CG_ROLL_LOOKS (1u << 14)
+#define CG_RESIDENT_LOOKS (1u << 21)
+
+// DevState::roll: blocks that have answered the call, and
+#define CG_ROLL_COUNT 0x0000ffffu
+#define CG_ROLL_LOST 0x40000000u       // a wait of an exchange ran out
+#define CG_ROLL_ENDED 0x20000000u      // block 0 has written the outcome
+
+// Whether all `blocks` blocks run; by one thread of each, to the same answer.
+__device__ __forceinline__ bool cg_roll_call(unsigned *roll, unsigned blocks, unsigned looks)
+{
+    unsigned v = atomicAdd(roll, 1u) + 1u;
+    for (unsigned k = 0;;) {
+        if (v & CG_ROLL_GIVEN_UP) return false;
+        if ((v & CG_ROLL_COUNT) == blocks) return true;
+        if (k++ < looks) {
+            __nanosleep(100);
+            v = *(volatile unsigned *)roll;
+        } else {
+            const unsigned was = atomicCAS(roll, v, v | CG_ROLL_GIVEN_UP);   // at most `blocks` times
+            v = was == v ? v | CG_ROLL_GIVEN_UP : was;
+        }
+    }
+}
 
 // (An exchange, not a store: a store reached the other blocks 2 us later, a
 // 32^3 iteration 11.8 us with a store, 11.2 with a fence after it, 10.2.)
@@ -52,10 +86,10 @@ __device__ __forceinline__ void cg_slot_get(const CgSlot *s, double &v, unsigned
 // (Up to 100 ns between two looks: without, the looks themselves cost a
 // system of two blocks a multiprocessor 0.5 to 1 us an iteration.)
 template <int NV>
-__device__ __forceinline__ bool cg_slot_wait(const CgSlot *s, bool mine, unsigned long long seq, double (&v)[NV])
+__device__ __forceinline__ bool cg_slot_wait(const CgSlot *s, bool mine, unsigned long long seq, double (&v)[NV],
+                                             unsigned looks)
 {
-    unsigned long long t0 = 0ull;
-    for (unsigned k = 1;; k++) {
+    for (unsigned k = 0;; k++) {
         unsigned long long got[NV];
         bool ok = true;
         if (mine) {
@@ -65,12 +99,8 @@ __device__ __forceinline__ bool cg_slot_wait(const CgSlot *s, bool mine, unsigne
             for (int j = 0; j < NV; j++) ok = ok && got[j] == seq;
         }
         if (__all_sync(FULL, ok)) return true;
+        if (k >= looks) return false;
         __nanosleep(100);
-        if ((k & 4095u) == 0u) {
-            const unsigned long long t = gtimer();
-            if (!t0) t0 = t;
-            if (__any_sync(FULL, t - t0 > CG_RESIDENT_WAIT_NS)) return false;
-        }
     }
 }
 
@@ -142,8 +172,13 @@ k_cg_resident(SellDev A, const double *__restrict__ val, Vec64 V, DevState *st, 
     __shared__ int s_run, s_lost;
     const int tid = threadIdx.x, G = gridDim.x, warps = G < TFS_TPB ? (G + 31) / 32 : TFS_TPB / 32;
     const int i = blockIdx.x * TFS_TPB + tid;
+    // tfs_diag_resident: the last block misses the call (1) or withholds its
+    // partial of the first exchange (2)
+    const int diag = blockIdx.x == G - 1 ? st->resident_diag : 0;
+    const unsigned looks = st->resident_looks ? st->resident_looks : CG_RESIDENT_LOOKS;
     if (tid == 0) {
-        s_run = st->done == 0;
+        s_run = st->done == 0 && diag != 1 &&
+                cg_roll_call(&st->roll, (unsigned)G, min(looks, CG_ROLL_LOOKS));
         s_lost = 0;
     }
     __syncthreads();
@@ -231,12 +266,12 @@ k_cg_resident(SellDev A, const double *__restrict__ val, Vec64 V, DevState *st, 
         {
             const double v[1] = {fma(p, q, 0.0)};
             const double s = cg_block_sum<1>(v, sm);
-            if (tid == 0) cg_slot_put(sq + blockIdx.x, s, seq);
+            if (tid == 0 && !(diag && it == 1)) cg_slot_put(sq + blockIdx.x, s, seq);
             double t[1] = {0.0};
             for (int b0 = tid & ~31; b0 < G; b0 += TFS_TPB) {
                 const int b = b0 + (tid & 31);
                 double u[1] = {0.0};
-                if (!cg_slot_wait<1>(sq + b, b < G, seq, u)) s_lost = 1;
+                if (!cg_slot_wait<1>(sq + b, b < G, seq, u, looks)) s_lost = 1;
                 t[0] = t[0] + u[0];
             }
             __syncthreads();
@@ -264,7 +299,7 @@ k_cg_resident(SellDev A, const double *__restrict__ val, Vec64 V, DevState *st, 
             for (int b0 = tid & ~31; b0 < G; b0 += TFS_TPB) {
                 const int b = b0 + (tid & 31);
                 double u[2] = {0.0, 0.0};
-                if (!cg_slot_wait<2>(sz + 2 * b, b < G, seq, u)) s_lost = 1;
+                if (!cg_slot_wait<2>(sz + 2 * b, b < G, seq, u, looks)) s_lost = 1;
                 t[0] = t[0] + u[0];
                 t[1] = t[1] + u[1];
             }
@@ -279,29 +314,43 @@ k_cg_resident(SellDev A, const double *__restrict__ val, Vec64 V, DevState *st, 
     }
     V.x[i] = x;
     V.r[i] = r;
-    if (s_lost) {                  // a wait ran out; every block finds the same
-        if (tid == 0) {
-            st->done = 1;
-            st->status = TFS_ERR_TIMEOUT;
-            st->niter_out = it + 1;
-            st->loops = loops;
-            *epoch = e0 + 2ull * (unsigned)loop_limit + 8ull;
-        }
-    } else if (blockIdx.x == 0) {
+    // The outcome: block 0's, unless a wait of any block ran out.  Others may
+    // not have found the same (in the last exchange a block can miss the others'
+    // partials after it has put its own): whichever of the two comes last at
+    // the roll word sees the other there and leaves the error standing.
+    bool lost = s_lost != 0;
+    if (blockIdx.x == 0 && !lost) {
         if (tid == 32) {
             st->error = err;
             st->fin_res = err;
             st->status = status;
             st->niter_out = niter_out;
             st->iter = it - 1;
-            st->loops = loops;
-            st->done = 1;
         }
         if (tid == 0) {
+            st->loops = loops;
             st->alpha = alfa;
             st->spmv_ns = spmv_ns;
             st->spmv_n = loops;
-            *epoch = e0 + 2ull * (unsigned)loop_limit + 8ull;
+        }
+        __syncthreads();
+    }
+    if (tid == 0) {
+        if (blockIdx.x == 0 && !lost) {
+            __threadfence();
+            lost = (atomicOr(&st->roll, CG_ROLL_ENDED) & CG_ROLL_LOST) != 0;
+        } else if (lost) {
+            atomicOr(&st->roll, CG_ROLL_LOST);
+        }
+        if (lost) {
+            __threadfence();
+            st->status = TFS_ERR_TIMEOUT;
+            st->niter_out = it + 1;
+            st->loops = loops;
+        }
+        if (lost || blockIdx.x == 0) {
+            st->done = 1;
+            atomicMax(epoch, e0 + 2ull * (unsigned)loop_limit + 8ull);
         }
     }
 }

@@ -342,7 +342,7 @@ static bool use_cg_resident(const tfs_handle *h, int method, int prec)
 {
     if (method != TFS_CG || prec == 2 || h->precision == TFS_MIXED || h->no_resident) return false;
     if (h->row_max > 8 || h->n_chunks > TFS_RESIDENT_CHUNKS) return false;
-    if (h->grid != h->n_chunks || h->grid_spmv != h->n_chunks || h->tile_room != INT64_MAX) return false;
+    if (h->grid != h->n_chunks || h->grid_spmv != h->n_chunks || h->served) return false;
     int per_sm = 0;
     const cudaError_t e = h->row_max <= 4
         ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg_resident<4>, TFS_TPB, 0)
@@ -952,6 +952,17 @@ extern "C" int tfs_diag_dic_timeout(tfs_handle *h, long long wait_ns)
         return TFS_ERR_ARG;
     }
     h->dicb_diag_ns = (unsigned long long)wait_ns;
+    return TFS_OK;
+}
+
+extern "C" int tfs_diag_resident(tfs_handle *h, int what, int looks)
+{
+    if (!h || what < 0 || what > 2 || looks < 0 || (what && !looks)) {
+        tfs_set_error_text("tfs_diag_resident: null handle, what outside 0..2 or no limit of the looks");
+        return TFS_ERR_ARG;
+    }
+    h->diag_resident = what;
+    h->diag_looks = looks;
     return TFS_OK;
 }
 
@@ -1748,7 +1759,7 @@ static int get_graph(tfs_handle *h, int method, int prec, GraphEntry **out)
         *out = &eager_entry;
         return TFS_OK;
     }
-    int key = method | (prec << 4) | (h->precision << 8);
+    const int key = method | (prec << 4) | (h->precision << 8) | (h->no_resident << 12);
     auto it = h->graphs.find(key);
     if (it != h->graphs.end()) { *out = &it->second; return TFS_OK; }
     GraphEntry ge;
@@ -1807,6 +1818,8 @@ int tfs_solve_launch(int method, tfs_handle *h, const double *val, double *x, do
     P.x = device_ptrs ? x : h->stage_x;
     P.r_out = device_ptrs ? r1 : h->stage_b;
     P.dicb_wait_ns = h->dicb_diag_ns;
+    P.resident_diag = h->diag_resident;
+    P.resident_looks = (unsigned)h->diag_looks;
     CK(cudaMemcpyAsync(h->params, h->h_params, sizeof(DevParams), cudaMemcpyHostToDevice, s));
     if (!device_ptrs) {
         CK(cudaMemcpyAsync(h->stage_val, val, sizeof(double) * (size_t)h->nnz, cudaMemcpyHostToDevice, s));
@@ -1866,6 +1879,15 @@ static int solve_impl(int method, tfs_handle *h, const double *val, double *x, d
     int rc = tfs_solve_launch(method, h, val, x, r1, prec, *niter, tol, device_ptrs);
     if (rc) return rc;
     CK(cudaStreamSynchronize(h->stream));
+    if (h->h_state->roll & CG_ROLL_GIVEN_UP) {
+        // Nothing is solved and nothing stored: the launched kernels.
+        const int keep = h->no_resident;
+        h->no_resident = 1;
+        rc = tfs_solve_launch(method, h, val, x, r1, prec, *niter, tol, device_ptrs);
+        h->no_resident = keep;
+        if (rc) return rc;
+        CK(cudaStreamSynchronize(h->stream));
+    }
     return tfs_solve_collect(h, niter, ini_res, fin_res);
 }
 
@@ -1967,6 +1989,8 @@ static int prepare_values(tfs_handle *h, const double *val, int prec = 0)
     P.x = h->stage_x;
     P.r_out = h->stage_b;
     P.dicb_wait_ns = 0;
+    P.resident_diag = 0;
+    P.resident_looks = 0;
     CK(cudaMemcpyAsync(h->params, h->h_params, sizeof(DevParams), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(h->stage_val, val, sizeof(double) * (size_t)h->nnz, cudaMemcpyHostToDevice, s));
     int gv = (h->nnz_pad + 255) / 256;

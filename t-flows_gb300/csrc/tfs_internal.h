@@ -32,6 +32,8 @@
 #define TFS_SPMV_DIRECT 0     // CG SpMV kernels: per-row dependent chain (any SELL-32 matrix)
 #define TFS_SPMV_PIPE 1       //   software-pipelined, uniform slice width
 
+#define CG_ROLL_GIVEN_UP 0x80000000u   // DevState::roll: k_cg_resident's roll call was given up
+
 // Device-resident state of one solve.  Written by k_init from DevParams and
 // then only by the last block of each reducing kernel.
 struct DevState {
@@ -43,7 +45,7 @@ struct DevState {
     int iter, done, niter_out, status;
     int early, loops, loop_limit, true_res;
     unsigned int counter;
-    unsigned int pad0;
+    unsigned int roll;   // k_cg_resident's roll call (CG_ROLL_*)
     unsigned long long t_spmv0, t_sweep0;
     unsigned long long spmv_ns, spmv_n, sweep_ns, sweep_n;
     // TFS_MIXED bookkeeping
@@ -68,6 +70,10 @@ struct DevState {
     // this many ns and its copy lane stages nothing (its first wait runs
     // out); 0, the normal limit
     unsigned long long dicb_wait_ns;
+    // tfs_diag_resident: what the last block leaves out, and the looks of a
+    // wait (0: the normal number)
+    int resident_diag;
+    unsigned int resident_looks;
 };
 
 // Per-call arguments, written by the host before every graph launch.
@@ -80,6 +86,8 @@ struct DevParams {
     double *x;               // natural order, n (in/out)
     double *r_out;           // natural order, n (r1 on return)
     unsigned long long dicb_wait_ns;   // DevState::dicb_wait_ns of the call
+    int resident_diag;                 // and DevState::resident_*
+    unsigned int resident_looks;
 };
 
 struct SellDev {
@@ -145,8 +153,10 @@ struct tfs_handle {
     int dic_tiles = 1;                 // TFS_OPT_DIC_TILES: 1 tiled DIC sweeps where the numbering allows
     TileStore *tiles[2] = {nullptr, nullptr};   // binary32, binary64 plan of the current layout (null: not made yet)
     int64_t tile_room = INT64_MAX;     // device bytes the plan may take (a server's budget)
+    bool served = false;               // a server's: other requests' kernels share the multiprocessors
     int tiles_used = 0;                // tiles of the last DIC application launched (0: none)
     unsigned long long dicb_diag_ns = 0;   // tfs_diag_dic_timeout
+    int diag_resident = 0, diag_looks = 0;   // tfs_diag_resident
     int diag_alloc = 0;                // tfs_diag_alloc_failure: the allocation that fails, counted down
     int l2_window = 1;                 // TFS_OPT_L2_WINDOW: 1 the column indices persisting in L2
     int dicb_used = 0;                 // the last DIC application launched was the one-block kernel

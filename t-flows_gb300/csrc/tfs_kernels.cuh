@@ -517,6 +517,8 @@ __global__ void k_init(DevState *st, const DevParams *prm, int prec)
     s.delta = 0.1;
     s.t_begin = gtimer();
     s.dicb_wait_ns = prm->dicb_wait_ns;
+    s.resident_diag = prm->resident_diag;
+    s.resident_looks = prm->resident_looks;
     *st = s;
 }
 
@@ -1403,6 +1405,7 @@ __global__ void k_store(int n_int, const int *__restrict__ perm, const double *_
                         const double *__restrict__ r, const DevParams *prm, DevState *st)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) st->t_end = gtimer();
+    if (st->roll & CG_ROLL_GIVEN_UP) return;   // nothing solved: x, r1 as they were for the next try
     double *xo = prm->x, *ro = prm->r_out;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_int; i += gridDim.x * blockDim.x) {
         int o = __ldg(perm + i);

@@ -147,6 +147,8 @@ static bool try_start(tfs_server *S, Request *r)
         // could use the slots (measured 232 against 252 solves/s on the
         // serving trace), so the server's handles launch them plainly.
         sy.h->pdl_vec = 0;
+        // (Nor does one request hold the multiprocessors for its whole solve.)
+        sy.h->served = true;
         // Nor do they mark their column indices persisting in L2: the
         // resident systems would compete for the one set-aside.
         sy.h->l2_window = 0;

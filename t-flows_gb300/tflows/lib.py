@@ -70,6 +70,7 @@ SIGNATURES = {
     "tfs_set_option": (C.c_int, [P_void, C.c_int, C.c_int]),
     "tfs_get_option": (C.c_int, [P_void, C.c_int, C.POINTER(C.c_int)]),
     "tfs_diag_dic_timeout": (C.c_int, [P_void, C.c_longlong]),
+    "tfs_diag_resident": (C.c_int, [P_void, C.c_int, C.c_int]),
     "tfs_diag_alloc_failure": (C.c_int, [P_void, C.c_int]),
     "tfs_solve": (C.c_int, [C.c_int, P_void, i32, i32, P_i32, P_i32, P_i32, P_dbl, P_dbl, P_dbl,
                             i32, P_i32, dbl, P_dbl, P_dbl]),
