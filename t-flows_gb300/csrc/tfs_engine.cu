@@ -1050,6 +1050,16 @@ static bool level_options_default(const tfs_handle *h)
 // memory's latency well before this.
 #define TFS_TILE_RING (96 << 10)
 
+// Whether sweeps of one vector in arithmetic T may go tile by tile: the option
+// and the layout, and a schedule that is neither deeper than the plans take nor
+// one of the deep narrow ones that fit the one-block DIC.
+template <typename T>
+static bool tiles_allowed(const tfs_handle *h)
+{
+    return h->dic_tiles && h->layout == TFS_LAYOUT_LEVELS && level_options_default(h) &&
+           h->n_levels <= TILE_MAX_LEVELS && !(h->n_levels >= TFS_DICB_SPLIT32_LEVELS && dic_block_kind<T>(h));
+}
+
 // The tiled DIC's plan for the current layout in values of T; tiles = 0 where
 // there is none, or the host has no memory for making it.
 template <typename T>
@@ -1128,7 +1138,7 @@ template <typename T>
 static int ensure_tiles(tfs_handle *h)
 {
     TileStore *&S = h->tiles[sizeof(T) == 8];
-    if (!h->dic_tiles || h->layout != TFS_LAYOUT_LEVELS || !level_options_default(h) || S) return TFS_OK;
+    if (!tiles_allowed<T>(h) || S) return TFS_OK;
     int optin = 0;
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
     CK(cudaFuncSetAttribute(k_dic_tile<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
@@ -1139,14 +1149,13 @@ static int ensure_tiles(tfs_handle *h)
     return upload_tiles(h, *S, P);
 }
 
-// Whether the sweeps of arithmetic T run tile by tile: a plan exists, and the
-// schedule is not one of the deep narrow ones that fit the one-block DIC.
+// Whether the sweeps of arithmetic T run tile by tile: they may, the entry point
+// sweeps one vector (sweep_tiles), and a plan exists.
 template <typename T>
 static bool use_tiles(const tfs_handle *h)
 {
     const TileStore *S = h->tiles[sizeof(T) == 8];
-    return h->dic_tiles && S && S->tiles > 0 && !h->profiling && level_options_default(h) &&
-           !(h->n_levels >= TFS_DICB_SPLIT32_LEVELS && dic_block_kind<T>(h));
+    return h->sweep_tiles && S && S->tiles > 0 && !h->profiling && tiles_allowed<T>(h);
 }
 
 template <typename T>
@@ -1637,7 +1646,7 @@ static int body_iterations(const tfs_handle *h, int method, int prec)
     if (prec != 2) return TFS_BODY_ITERATIONS;
     const bool mixed = h->precision == TFS_MIXED;
     const bool few = mixed ? use_tiles<float>(h) || dic_block_kind<float>(h) : use_tiles<double>(h) || dic_block_kind<double>(h);
-    return few && method != TFS_BICG ? TFS_BODY_ITERATIONS : 1;   // (the literal BiCG sweeps two vectors by levels)
+    return few && method != TFS_BICG ? TFS_BODY_ITERATIONS : 1;
 }
 
 static int build_graph(tfs_handle *h, int method, int prec, GraphEntry &ge)
@@ -1796,7 +1805,6 @@ int tfs_solve_launch(int method, tfs_handle *h, const double *val, double *x, do
     CK(cudaSetDevice(h->device));
     int rc = ensure_layout(h, prec);
     if (rc) return rc;
-    if (prec == 2 && (rc = h->precision == TFS_MIXED ? ensure_tiles<float>(h) : ensure_tiles<double>(h))) return rc;
     // The reference's BiCG starts its shadow residual as r1 and drives it
     // with A, not A^T (Bicg.f90:91-93, 107-108, 136-144, 171-175): the shadow
     // sequence equals the primary one bit for bit, rho = (z1, r2) = (r1, z1)
@@ -1804,6 +1812,8 @@ int tfs_solve_launch(int method, tfs_handle *h, const double *val, double *x, do
     // It therefore runs through the CG kernels (half the work, same bits);
     // TFS_OPT_BICG = 1 runs the two sequences explicitly.
     const int kmethod = (method == TFS_BICG && !h->bicg_literal) ? TFS_CG : method;
+    h->sweep_tiles = prec == 2 && kmethod != TFS_BICG;   // (the literal BiCG sweeps two vectors, by levels)
+    if (h->sweep_tiles && (rc = h->precision == TFS_MIXED ? ensure_tiles<float>(h) : ensure_tiles<double>(h))) return rc;
     GraphEntry *ge = nullptr;
     rc = get_graph(h, kmethod, prec, &ge);
     if (rc) return rc;
@@ -2018,11 +2028,12 @@ static int vec_out(tfs_handle *h, const double *src, double *host)
     return TFS_OK;
 }
 
-// The preconditioner of h->val, and for DIC the tiles' packed values in the
-// arithmetic that is going to sweep.
-static int form_prec(tfs_handle *h, int prec, int mode = TFS_FP64)
+// The preconditioner of h->val, and where DIC sweeps follow the tiles' packed
+// values in the arithmetic that is going to sweep.
+static int form_prec(tfs_handle *h, int prec, bool sweeps, int mode = TFS_FP64)
 {
-    if (prec == 2) {
+    h->sweep_tiles = prec == 2 && sweeps;
+    if (h->sweep_tiles) {
         int rc = mode == TFS_FP64 ? ensure_tiles<double>(h) : ensure_tiles<float>(h);
         if (rc) return rc;
     }
@@ -2065,7 +2076,7 @@ extern "C" int tfs_prec_form(tfs_handle *h, const double *val, int32_t prec, dou
     if (!h || !val || !d || prec < 0 || prec > 2) return TFS_ERR_ARG;
     CK(cudaSetDevice(h->device));
     int rc;
-    if ((rc = prepare_values(h, val, prec)) || (rc = form_prec(h, prec))) return rc;
+    if ((rc = prepare_values(h, val, prec)) || (rc = form_prec(h, prec, false))) return rc;
     return vec_out(h, h->v.d, d);
 }
 
@@ -2074,7 +2085,7 @@ extern "C" int tfs_prec_solve(tfs_handle *h, const double *val, int32_t prec, co
     if (!h || !val || !b || !x || prec < 0 || prec > 2) return TFS_ERR_ARG;
     CK(cudaSetDevice(h->device));
     int rc;
-    if ((rc = prepare_values(h, val, prec)) || (rc = form_prec(h, prec)) || (rc = vec_in(h, b, h->v.r))) return rc;
+    if ((rc = prepare_values(h, val, prec)) || (rc = form_prec(h, prec, true)) || (rc = vec_in(h, b, h->v.r))) return rc;
     if (prec == 2) {
         int cnt = 0;
         if ((rc = launch_sweeps<double>(h, h->stream, 1, h->v.r, nullptr, h->v.y, nullptr, h->v.z, nullptr, &cnt))) return rc;
@@ -2143,7 +2154,7 @@ extern "C" int tfs_time_prec(tfs_handle *h, const double *val, int mode, int rep
     CK(cudaSetDevice(h->device));
     int rc = prepare_values(h, val, 2);
     if (rc) return rc;
-    if ((rc = form_prec(h, 2, mode))) return rc;
+    if ((rc = form_prec(h, 2, true, mode))) return rc;
     SellDev A = sell_of(h);
     cudaStream_t s = h->stream;
     k_diag_form<<<(h->n_int + 255) / 256, 256, 0, s>>>(A, h->val, h->v.r, 0);

@@ -151,6 +151,7 @@ struct tfs_handle {
     int bicg_literal = 0;              // TFS_OPT_BICG: 1 BiCG runs its shadow sequence explicitly
     int dic_block = 1;                 // TFS_OPT_DIC_BLOCK: 1 one-block DIC where the vector and two slots of the widest level fit
     int dic_tiles = 1;                 // TFS_OPT_DIC_TILES: 1 tiled DIC sweeps where the numbering allows
+    bool sweep_tiles = false;          // the call at hand sweeps one vector, tile by tile where it can
     TileStore *tiles[2] = {nullptr, nullptr};   // binary32, binary64 plan of the current layout (null: not made yet)
     int64_t tile_room = INT64_MAX;     // device bytes the plan may take (a server's budget)
     bool served = false;               // a server's: other requests' kernels share the multiprocessors
