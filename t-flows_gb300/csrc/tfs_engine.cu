@@ -338,16 +338,18 @@ static cudaError_t launch_cg_resident(const tfs_handle *h, cudaStream_t s)
 // block resident, and not of a server, whose other requests' kernels share
 // the multiprocessors.  (Faster than the kernels of an iteration at every
 // size it can take.)
-static bool use_cg_resident(const tfs_handle *h, int method, int prec)
+static bool use_cg_resident(tfs_handle *h, int method, int prec)
 {
     if (method != TFS_CG || prec == 2 || h->precision == TFS_MIXED || h->no_resident) return false;
     if (h->row_max > 8 || h->n_chunks > TFS_RESIDENT_CHUNKS) return false;
     if (h->grid != h->n_chunks || h->grid_spmv != h->n_chunks || h->served) return false;
-    int per_sm = 0;
-    const cudaError_t e = h->row_max <= 4
-        ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg_resident<4>, TFS_TPB, 0)
-        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg_resident<8>, TFS_TPB, 0);
-    return e == cudaSuccess && h->n_chunks <= per_sm * h->sm_count;
+    if (h->resident_per_sm < 0) {
+        const cudaError_t e = h->row_max <= 4
+            ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&h->resident_per_sm, k_cg_resident<4>, TFS_TPB, 0)
+            : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&h->resident_per_sm, k_cg_resident<8>, TFS_TPB, 0);
+        if (e != cudaSuccess) h->resident_per_sm = 0;
+    }
+    return h->n_chunks <= h->resident_per_sm * h->sm_count;
 }
 
 static uint64_t fingerprint(int32_t n, int32_t nnz, const int32_t *row1, const int32_t *col1,
@@ -662,6 +664,7 @@ static int build_layout(tfs_handle *h, int kind)
     // TFS_OPT_SELL_UNIFORM = 0 keeps per-slice widths.
     h->sell_width = 0;
     h->row_max = wmax;
+    h->resident_per_sm = -1;
     {
         const int64_t uni = 32 * (int64_t)wmax * n_slices;
         if (h->sell_uniform && wmax > 0 && wmax <= 8 && uni <= off + off / 20 && uni <= INT32_MAX) {
@@ -1637,19 +1640,45 @@ static void l2_window_nodes(cudaGraph_t g, const cudaAccessPolicyWindow &w)
     }
 }
 
+// A loop body of few kernels holds TFS_BODY_ITERATIONS iterations: going round
+// the loop costs 4 to 5 us (a 32^3 diagonal CG iteration 21.2 -> 17.4 us, a
+// 64^3 DIC-CG iteration 55.3 -> 51.2 mixed).  Kernels past the end of the solve
+// return at once, at 4 (diagonal) to 13 us (tiled DIC) for each iteration that
+// the last body has too many, so solves that are expected to be short go
+// singly: 32^3 mixed, diagonal, 1, 2 and 5 iterations 82, 104 and 166 us, in
+// bodies of four 95, 107 and 166; 1,320 rows, DIC, 119, 157 and 279 against 142,
+// 169 and 293.  From TFS_BODIES_FROM on the rounds saved outweigh the three
+// iterations too many at most.  (Three kinds of body in one graph, singles
+// before and after, cost every solve the 10 us of another conditional node.
+// The mixed solves' true-residual step stays with every iteration: once a body
+// it saved two idle kernels, 4 us, an iteration of a slow solve, but a fast
+// one, which asks for it every iteration or two, then leaves most of each body
+// idle.)
 #define TFS_BODY_ITERATIONS 4
+#define TFS_BODIES_FROM 12
 
-// Iterations of a loop body: TFS_BODY_ITERATIONS unless the sweeps are
-// launched level by level.
-static int body_iterations(const tfs_handle *h, int method, int prec)
+// The iterations that a solve is expected to take: its limit, or what the last
+// solve of the kind (key) on this handle took to its tolerance, if that is
+// fewer.  It decides how the kernels are launched, never what they compute.
+static int expected_iterations(const tfs_handle *h, int key, int niter)
 {
+    const auto last = h->last_loops.find(key);
+    return last == h->last_loops.end() ? niter : std::min(niter, last->second);
+}
+
+// Iterations of a loop body: one where few are expected or the sweeps are
+// launched level by level (many kernels, whose idle launches would cost more
+// than going round).
+static int body_iterations(tfs_handle *h, int method, int prec, int expected)
+{
+    if (expected < TFS_BODIES_FROM || use_cg_resident(h, method, prec)) return 1;
     if (prec != 2) return TFS_BODY_ITERATIONS;
     const bool mixed = h->precision == TFS_MIXED;
     const bool few = mixed ? use_tiles<float>(h) || dic_block_kind<float>(h) : use_tiles<double>(h) || dic_block_kind<double>(h);
     return few && method != TFS_BICG ? TFS_BODY_ITERATIONS : 1;
 }
 
-static int build_graph(tfs_handle *h, int method, int prec, GraphEntry &ge)
+static int build_graph(tfs_handle *h, int method, int prec, int reps, GraphEntry &ge)
 {
     const cudaAccessPolicyWindow l2w = l2_window_of(h);
     l2_window_streams(h, l2w);
@@ -1697,15 +1726,6 @@ static int build_graph(tfs_handle *h, int method, int prec, GraphEntry &ge)
         // Body, captured on the second stream into the conditional node's graph.
         e = cudaStreamBeginCaptureToGraph(h->stream2, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return fail(e, "begin body capture");
-        // A body of few kernels holds TFS_BODY_ITERATIONS iterations: going round
-        // the loop costs 4 to 5 us (a 32^3 diagonal CG iteration 21.2 -> 17.4 us,
-        // a 64^3 DIC-CG iteration 55.3 -> 51.2 mixed).  Kernels past the end of
-        // the solve return at once; a body of many (level kernels) would lose
-        // more to those than it gains.  (The mixed solves' true-residual step
-        // stays with every iteration: once a body it saved two idle kernels, 4 us,
-        // an iteration of a slow solve, but a fast one, which asks for it every
-        // iteration or two, then leaves most of each body idle.)
-        const int reps = body_iterations(h, method, prec);
         for (int k = 0; k < reps && !rc; k++) {
             if (h->precision == TFS_MIXED) rc = tfs_mixed_body(h, h->stream2, method, prec, cond, &ge.body_kernels);
             else rc = launch_body(h, h->stream2, method, prec, cond, &ge.body_kernels);
@@ -1761,33 +1781,37 @@ static int run_eager(tfs_handle *h, int method, int prec, GraphEntry *ge)
     return TFS_OK;
 }
 
-static int get_graph(tfs_handle *h, int method, int prec, GraphEntry **out)
+// The kind of solve: method, preconditioner and arithmetic.
+static int solve_key(const tfs_handle *h, int method, int prec) { return method | (prec << 4) | (h->precision << 8); }
+
+static int get_graph(tfs_handle *h, int method, int prec, int expected, GraphEntry **out)
 {
     if (h->eager) {
         static thread_local GraphEntry eager_entry;
         *out = &eager_entry;
         return TFS_OK;
     }
-    const int key = method | (prec << 4) | (h->precision << 8) | (h->no_resident << 12);
-    auto it = h->graphs.find(key);
+    const int reps = body_iterations(h, method, prec, expected);
+    auto key = [&] { return solve_key(h, method, prec) | (h->no_resident << 12) | ((reps > 1) << 13); };
+    auto it = h->graphs.find(key());
     if (it != h->graphs.end()) { *out = &it->second; return TFS_OK; }
     GraphEntry ge;
-    int rc = build_graph(h, method, prec, ge);
+    int rc = build_graph(h, method, prec, reps, ge);
     if (rc && use_cg_resident(h, method, prec)) {
         // A driver that cannot hold a cooperative launch in a graph.
         h->no_resident = 1;
         ge = GraphEntry();
-        rc = build_graph(h, method, prec, ge);
+        rc = build_graph(h, method, prec, reps, ge);
     }
     if (rc && h->use_pdl) {
         // A driver that cannot keep programmatic edges inside a conditional
         // body gets plain stream-ordered level launches instead.
         h->use_pdl = 0;
-        rc = build_graph(h, method, prec, ge);
+        rc = build_graph(h, method, prec, reps, ge);
     }
     if (rc) return rc;
-    h->graphs[key] = ge;
-    *out = &h->graphs[key];
+    h->graphs[key()] = ge;
+    *out = &h->graphs[key()];
     return TFS_OK;
 }
 
@@ -1815,7 +1839,8 @@ int tfs_solve_launch(int method, tfs_handle *h, const double *val, double *x, do
     h->sweep_tiles = prec == 2 && kmethod != TFS_BICG;   // (the literal BiCG sweeps two vectors, by levels)
     if (h->sweep_tiles && (rc = h->precision == TFS_MIXED ? ensure_tiles<float>(h) : ensure_tiles<double>(h))) return rc;
     GraphEntry *ge = nullptr;
-    rc = get_graph(h, kmethod, prec, &ge);
+    h->last_key = solve_key(h, kmethod, prec);
+    rc = get_graph(h, kmethod, prec, expected_iterations(h, h->last_key, niter), &ge);
     if (rc) return rc;
     h->last_graph = ge;
     cudaStream_t s = h->stream;
@@ -1861,6 +1886,7 @@ int tfs_solve_launch(int method, tfs_handle *h, const double *val, double *x, do
 int tfs_solve_collect(tfs_handle *h, int32_t *niter, double *ini_res, double *fin_res)
 {
     const DevState &S = *h->h_state;
+    h->last_loops[h->last_key] = S.niter_out > S.niter_max ? INT32_MAX : S.loops;
     if (S.early != 1) *ini_res = S.ini_res;
     *fin_res = S.fin_res;
     *niter = S.niter_out;

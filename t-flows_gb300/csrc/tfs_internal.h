@@ -129,6 +129,7 @@ struct tfs_handle {
     int n_int = 0, n_chunks = 0, n_slices = 0, nnz_pad = 0, n_levels = 0;
     int sell_width = 0;                // uniform slice width (0: per-slice widths)
     int row_max = 0;                   // entries of the longest row
+    int resident_per_sm = -1;          // blocks of k_cg_resident a multiprocessor holds (-1: not asked yet)
     int no_resident = 0;               // k_cg_resident could not be captured
     int spmv_kind = 0;                 // TFS_SPMV_DIRECT / _PIPE: kernel of the CG SpMV
     int grid = 0;                      // blocks of the vector kernels (grid-stride)
@@ -200,7 +201,9 @@ struct tfs_handle {
     // pinned host mirror of params and state
     DevParams *h_params = nullptr;
     DevState *h_state = nullptr;
-    std::map<int, GraphEntry> graphs;  // key: method | prec << 4 | precision << 8
+    std::map<int, GraphEntry> graphs;  // by kind (solve_key) and how it is launched (get_graph)
+    std::map<int, int> last_loops;     // iterations of the last solve of each kind (solve_key), INT32_MAX: its limit
+    int last_key = 0;                  // kind of the last solve launched
     tfs_stats stats{};
     int64_t device_bytes = 0;
     FaceMap *faces = nullptr;          // tfs_faces_register

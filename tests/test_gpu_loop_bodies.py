@@ -1,0 +1,42 @@
+"""Loop bodies of one iteration or of four, whichever the solve is expected to
+fill: whatever came before on the handle, every solve gives the bits of the same
+solve launched kernel by kernel on a handle of its own."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from helpers import system
+from tflows import TFS_BICG, TFS_CG, TFS_CGS, TFS_FP64, TFS_MIXED, Solver
+from tflows.lib import TFS_OPT_BICG, TFS_OPT_LAUNCH
+from tflows.synth import CONVDIFF, POISSON
+
+pytestmark = pytest.mark.gpu
+
+# (limit, relative tolerance): long and short in turn, ended by either
+SERIES = [(40, 1e-30), (1, 1e-30), (2, 1e-30), (3000, 0.5), (3000, 1e-6), (13, 1e-30), (11, 1e-30), (3000, 0.2),
+          (0, 1e-6), (3000, 1e-3), (5, 1e-30), (3000, 2.0), (3000, 1e-2), (12, 1e-30), (3, 1e-30), (3000, 1e-4)]
+
+
+def _solve(sol, s, method, prec, limit, rel):
+    x, r = np.zeros(s.n), s.b.copy()
+    res = sol.solve(method, s.val, x, r, prec, limit, rel * float(np.linalg.norm(s.b)))
+    return [x, r, np.array([res.niter, res.status, sol.stats()["iterations"]]), np.array([res.ini_res, res.fin_res])]
+
+
+@pytest.mark.parametrize("kind,shape,permute,method,literal", [
+    (POISSON, (12, 11, 10), True, TFS_CG, 0), (POISSON, (30, 28, 26), True, TFS_CG, 0),
+    (POISSON, (14, 13, 12), False, TFS_CG, 0), (POISSON, (50, 50, 50), True, TFS_CG, 0),
+    (CONVDIFF, (20, 20, 20), True, TFS_CGS, 0), (POISSON, (16, 15, 14), True, TFS_BICG, 1)])
+@pytest.mark.parametrize("mode", [TFS_FP64, TFS_MIXED])
+@pytest.mark.parametrize("prec", [1, 2])
+def test_bodies_whatever_came_before(kind, shape, permute, method, literal, mode, prec, gpu):
+    s = system(kind, *shape, permute=permute)
+    opts = {TFS_OPT_BICG: literal}
+    with Solver(s.matrix(), precision=mode, options={**opts, TFS_OPT_LAUNCH: 1}) as sol:
+        want = [_solve(sol, s, method, prec, n, rel) for n, rel in SERIES]
+    with Solver(s.matrix(), precision=mode, options=opts) as sol:
+        for _ in range(2):
+            for (n, rel), w in zip(SERIES, want, strict=True):
+                for a, b in zip(_solve(sol, s, method, prec, n, rel), w, strict=True):
+                    assert np.array_equal(a, b), (n, rel)
