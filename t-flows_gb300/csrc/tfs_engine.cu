@@ -1796,11 +1796,13 @@ static int get_graph(tfs_handle *h, int method, int prec, int expected, GraphEnt
     auto it = h->graphs.find(key());
     if (it != h->graphs.end()) { *out = &it->second; return TFS_OK; }
     GraphEntry ge;
+    ge.reps = reps;
     int rc = build_graph(h, method, prec, reps, ge);
     if (rc && use_cg_resident(h, method, prec)) {
         // A driver that cannot hold a cooperative launch in a graph.
         h->no_resident = 1;
         ge = GraphEntry();
+        ge.reps = reps;
         rc = build_graph(h, method, prec, reps, ge);
     }
     if (rc && h->use_pdl) {
@@ -1902,7 +1904,9 @@ int tfs_solve_collect(tfs_handle *h, int32_t *niter, double *ini_res, double *fi
     T.sweep_ns_total = (double)S.sweep_ns;
     T.sweep_launches = (int64_t)S.sweep_n;
     const GraphEntry *ge = h->last_graph;
-    T.kernel_launches = ge ? ge->prologue_kernels + (int64_t)S.loops * ge->body_kernels + ge->epilogue_kernels : 0;
+    // (whole bodies: the iterations past the end of the solve are launched too)
+    const int64_t its = ge ? (S.loops + ge->reps - 1) / ge->reps * (int64_t)ge->reps : 0;
+    T.kernel_launches = ge ? ge->prologue_kernels + its * ge->body_kernels + ge->epilogue_kernels : 0;
     T.device_bytes = h->device_bytes;
     return S.status;
 }

@@ -115,7 +115,8 @@ struct TileStore; // tfs_engine.cu: the tiled DIC's plan on the device
 struct GraphEntry {
     cudaGraphExec_t exec = nullptr;
     cudaGraph_t graph = nullptr;
-    int prologue_kernels = 0, body_kernels = 0, epilogue_kernels = 0;
+    int prologue_kernels = 0, body_kernels = 0, epilogue_kernels = 0;   // (body: of one iteration)
+    int reps = 1;                        // iterations of a body
     int dic_kernel = 0, dic_tiles = 0;   // of its sweeps: tfs_handle::dicb_used, tiles_used
 };
 

@@ -40,3 +40,28 @@ def test_bodies_whatever_came_before(kind, shape, permute, method, literal, mode
             for (n, rel), w in zip(SERIES, want, strict=True):
                 for a, b in zip(_solve(sol, s, method, prec, n, rel), w, strict=True):
                     assert np.array_equal(a, b), (n, rel)
+
+
+@pytest.mark.parametrize("mode,prec", [(TFS_MIXED, 1), (TFS_FP64, 2)])
+def test_kernel_launches_count_whole_bodies(mode, prec, gpu):
+    """A solve's launches: those around the loop and an iteration's, times the
+    iterations launched -- in bodies of four also those past the solve's end."""
+    s = system(POISSON, 30, 28, 26)
+
+    def count(sol, limit, rel):
+        it = _solve(sol, s, TFS_CG, prec, limit, rel)[2][2]
+        return it, sol.stats()["kernel_launches"]
+
+    with Solver(s.matrix(), precision=mode) as sol:
+        assert count(sol, 0, 1e-30)[0] == 0
+        around = sol.stats()["kernel_launches"]
+        one = count(sol, 1, 1e-30)[1] - around
+        assert one >= 3 and count(sol, 7, 1e-30) == (7, around + 7 * one)       # singly
+        for limit in (12, 13, 14, 40, 41):
+            assert count(sol, limit, 1e-30) == (limit, around + (limit + 3) // 4 * 4 * one)
+        seen = set()
+        for rel in (1e-3, 1e-4, 1e-5, 1e-6):
+            it, launched = count(sol, 3000, rel)
+            assert it >= 12 and launched == around + (it + 3) // 4 * 4 * one
+            seen.add(it % 4)
+        assert seen - {0}
