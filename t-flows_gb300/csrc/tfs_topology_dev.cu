@@ -32,7 +32,10 @@
 // with the searches (600 without the cache hints).
 //
 // The faces must join distinct pairs of distinct cells (each stored entry
-// then belongs to exactly one face side), as meshes from the reference's
+// then belongs to exactly one face side; where several faces join a pair all
+// the same, every one of its entries gets the pair's first place as mir and
+// every face its last as pos, as row searches give them), as meshes from the
+// reference's
 // generators do; every array is 1-based, as in the reference.
 #include <cuda_runtime.h>
 
@@ -52,11 +55,12 @@ constexpr int kRowMax = 8;     // entries of a row sorted in registers
 // nothing: cudaMalloc and cudaFree took up to 0.2 ms of it.
 struct TopoState {
     int bad, total;
+    int twice;        // a pair of cells is joined by more than one face
 };
 __device__ TopoState g_topo;
 std::mutex g_topo_mutex;
 
-__global__ void k_topo_reset() { g_topo = TopoState{0, 0}; }
+__global__ void k_topo_reset() { g_topo = TopoState{0, 0, 0}; }
 
 __global__ void k_topo_zero(int n, int *width)
 {
@@ -204,9 +208,11 @@ k_topo_sort(int n_cells, const int *__restrict__ fc, const int *__restrict__ row
                     col1[k + 1] = v;
                     side[k + 1] = w;
                 }
-                for (int p = b; p < e; p++) {
+                for (int p = e - 1, last = e; p >= b; p--) {   // last: of the entries of this column
+                    if (p + 1 < e && col1[p] == col1[p + 1]) g_topo.twice = 1;
+                    else last = p + 1;
                     if (side[p] < 0) dia1[c] = p + 1;
-                    else pos1[side[p]] = p + 1;
+                    else pos1[side[p]] = last;
                 }
             }
             __syncthreads();
@@ -233,6 +239,7 @@ k_topo_sort(int n_cells, const int *__restrict__ fc, const int *__restrict__ row
                         v[q + 1] = tv;
                         w[q + 1] = tw;
                     }
+            bool twice = false;
 #pragma unroll
             for (int q = 0; q < kRowMax; q++)
                 if (q < len) {
@@ -240,7 +247,15 @@ k_topo_sort(int n_cells, const int *__restrict__ fc, const int *__restrict__ row
                     ss[b - first + q] = w[q];
                     if (w[q] < 0) dia1[c] = b + q + 1;
                     else pos1[w[q]] = b + q + 1;
+                    if (q > 0) twice = twice || v[q] == v[q - 1];
                 }
+            if (twice) {
+                g_topo.twice = 1;
+                for (int q = len - 2, last = len; q >= 0; q--) {
+                    if (sc[b - first + q] != sc[b - first + q + 1]) last = q + 1;
+                    if (ss[b - first + q] >= 0) pos1[ss[b - first + q]] = b + last;
+                }
+            }
         }
         __syncthreads();
         for (int p = first + threadIdx.x; p < end; p += kTB) {
@@ -252,14 +267,19 @@ k_topo_sort(int n_cells, const int *__restrict__ fc, const int *__restrict__ row
 }
 
 // mir(p) in place of the entry's face side: the position of the same face's
-// other entry, or the diagonal's own.
-__global__ void k_topo_mir(const int *__restrict__ pos1, int *mir1)
+// other entry (the first of its pair), or the diagonal's own.
+__global__ void k_topo_mir(const int *__restrict__ pos1, const int *__restrict__ row1, const int *__restrict__ col1,
+                           int *mir1)
 {
     if (g_topo.bad) return;
     const int n = g_topo.total;
+    const bool twice = g_topo.twice != 0;
     for (int p = blockIdx.x * kTB + threadIdx.x; p < n; p += gridDim.x * kTB) {
         const int s = __ldcs(mir1 + p);
-        __stcs(mir1 + p, s < 0 ? p + 1 : __ldg(pos1 + (s ^ 1)));
+        int m = s < 0 ? p + 1 : __ldg(pos1 + (s ^ 1));
+        if (twice && s >= 0)
+            for (const int row = __ldg(row1 + __ldg(col1 + p) - 1); m > row && col1[m - 2] == col1[m - 1];) m--;
+        __stcs(mir1 + p, m);
     }
 }
 
@@ -308,9 +328,9 @@ extern "C" int tfs_topology_build_device(int32_t n_cells, int32_t n_faces, const
     k_scan_add<<<grid((int64_t)n_cells + 1), kTB>>>(n_cells, bsum, d_row1);
     if (n_faces > 0) k_topo_fill<<<grid(n_faces), kTB>>>(n_faces, d_faces_c, d_pos1, d_row1, d_mir1);
     k_topo_sort<<<grid(n_cells), kTB>>>(n_cells, d_faces_c, d_row1, d_col1, d_mir1, d_dia1, d_pos1);
-    k_topo_mir<<<grid((int64_t)n_cells + 2 * (int64_t)n_faces), kTB>>>(d_pos1, d_mir1);
+    k_topo_mir<<<grid((int64_t)n_cells + 2 * (int64_t)n_faces), kTB>>>(d_pos1, d_row1, d_col1, d_mir1);
     e = cudaGetLastError();
-    TopoState out{0, 0};
+    TopoState out{0, 0, 0};
     if (e == cudaSuccess) e = cudaMemcpyFromSymbol(&out, g_topo, sizeof out);
     if (e != cudaSuccess) return tfs_engine_error(e, "tfs_topology_build_device");
     if (out.bad) {
