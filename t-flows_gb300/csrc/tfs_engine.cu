@@ -1066,17 +1066,18 @@ static bool tiles_allowed(const tfs_handle *h)
 // The tiled DIC's plan for the current layout in values of T; tiles = 0 where
 // there is none, or the host has no memory for making it.
 template <typename T>
-static TilePlan make_tiles(const tfs_handle *h, int optin)
+static TilePlan make_tiles(tfs_handle *h, int optin)
 {
     TilePlan P;
     try {
+        if (!h->tile_part) h->tile_part = std::make_shared<TilePartition>();
         const int threads = std::max(1, std::min(16, (int)std::thread::hardware_concurrency()));
         std::vector<int> internal(h->n);
         for (int k = 0; k < h->n_int; k++)
             if (h->perm_host[k] >= 0) internal[h->perm_host[k]] = k;
         for (int tries = 0, tiles = tile_count(h->n, h->sm_count); tries < 2 && !P.tiles; tries++, tiles += h->sm_count)
             P = tile_plan(h->n, h->row0, h->col0, h->dia0, h->levels_nat, h->rcm_pos, internal, tiles,
-                          TFS_TILE_MAX_RATIO, sizeof(T), optin, TFS_TILE_RING, threads);
+                          TFS_TILE_MAX_RATIO, sizeof(T), optin, TFS_TILE_RING, threads, h->tile_part.get());
     } catch (const std::exception &) {
         P.tiles = 0;
     }

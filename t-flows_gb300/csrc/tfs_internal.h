@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <map>
+#include <memory>
 #include <vector>
 
 #include "../../include/tfs_solver.h"
@@ -111,6 +112,7 @@ struct Vec32 {
 
 struct FaceMap;   // tfs_assemble.cu
 struct TileStore; // tfs_engine.cu: the tiled DIC's plan on the device
+namespace tfs { struct TilePartition; }   // tfs_dic_tiles_plan.h
 
 struct GraphEntry {
     cudaGraphExec_t exec = nullptr;
@@ -154,6 +156,7 @@ struct tfs_handle {
     int dic_block = 1;                 // TFS_OPT_DIC_BLOCK: 1 one-block DIC where the vector and two slots of the widest level fit
     int dic_tiles = 1;                 // TFS_OPT_DIC_TILES: 1 tiled DIC sweeps where the numbering allows
     bool sweep_tiles = false;          // the call at hand sweeps one vector, tile by tile where it can
+    std::shared_ptr<tfs::TilePartition> tile_part;   // of the plan made last, for the other arithmetic's
     TileStore *tiles[2] = {nullptr, nullptr};   // binary32, binary64 plan of the current layout (null: not made yet)
     int64_t tile_room = INT64_MAX;     // device bytes the plan may take (a server's budget)
     bool served = false;               // a server's: other requests' kernels share the multiprocessors
