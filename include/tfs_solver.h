@@ -170,9 +170,11 @@ int tfs_set_default_precision(int mode);
 #define TFS_OPT_DIC_TILES    16  /* 1 DIC sweeps tile by tile, each tile with the
                                     rows it depends on in one block's shared
                                     memory, where the cell numbering keeps those
-                                    few (default; not where TFS_OPT_TAIL_PF,
-                                    _FWD_PRE or _BWD_PRE are 0); 0 the level
-                                    kernels                                     */
+                                    few (not where TFS_OPT_TAIL_PF, _FWD_PRE or
+                                    _BWD_PRE are 0); 2 the same where it is the
+                                    faster way for the system's size and the
+                                    iterations a solve is expected to take
+                                    (default); 0 the level kernels              */
 
 /* One DIC application (the tfs_time_prec workload: factor from val, r = 1)
  * with its level launches stamped on the device: for slot k (launch order)

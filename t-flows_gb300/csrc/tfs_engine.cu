@@ -902,7 +902,7 @@ static void drop_graphs(tfs_handle *h)
 static int *option_field(tfs_handle *h, int option, bool (**ok)(int))
 {
     static bool (*const bit)(int) = [](int v) { return v == 0 || v == 1; };
-    static bool (*const fuse)(int) = [](int v) { return v >= 0 && v <= 2; };
+    static bool (*const three)(int) = [](int v) { return v >= 0 && v <= 2; };
     static bool (*const tpb)(int) = [](int v) { return v == 128 || v == 256 || v == 512 || v == 1024; };
     *ok = bit;
     switch (option) {
@@ -914,14 +914,14 @@ static int *option_field(tfs_handle *h, int option, bool (**ok)(int))
     case TFS_OPT_SPMV_GRID: return &h->spmv_chunks;
     case TFS_OPT_LEVEL_TPB: *ok = tpb; return &h->level_tpb;
     case TFS_OPT_TAIL_PF: return &h->tail_pf;
-    case TFS_OPT_FUSE_L0: *ok = fuse; return &h->fuse_l0;
+    case TFS_OPT_FUSE_L0: *ok = three; return &h->fuse_l0;
     case TFS_OPT_PDL: return &h->use_pdl;
     case TFS_OPT_PDL_VEC: return &h->pdl_vec;
     case TFS_OPT_FWD_PRE: return &h->fwd_pre;
     case TFS_OPT_BWD_PRE: return &h->bwd_pre;
     case TFS_OPT_DIC_BLOCK: return &h->dic_block;
     case TFS_OPT_L2_WINDOW: return &h->l2_window;
-    case TFS_OPT_DIC_TILES: return &h->dic_tiles;
+    case TFS_OPT_DIC_TILES: *ok = three; return &h->dic_tiles;
     default: return nullptr;
     }
 }
@@ -1063,6 +1063,42 @@ static bool tiles_allowed(const tfs_handle *h)
            h->n_levels <= TILE_MAX_LEVELS && !(h->n_levels >= TFS_DICB_SPLIT32_LEVELS && dic_block_kind<T>(h));
 }
 
+// Whether tiles are also the faster way for a solve expected to take so many
+// iterations (TFS_OPT_DIC_TILES = 2; 1 sweeps by them wherever there is a plan).
+//   - Small systems stay with the one-block DIC where it takes them: two tile
+//     launches cost more than its one.  A solve of 40 iterations, us, one block
+//     / tiles, binary32: 512 rows 1520 / 1631, 1,320 1656 / 1732, 2,940 1781 /
+//     1802, 3,150 1774 / 1734, 4,096 1938 / 1795; binary64: 512 1581 / 1594,
+//     1,320 2159 / 2073, 2,028 2333 / 2148.
+//   - A solve packs the values first, which comes back after more iterations
+//     the larger the system is.  Tiles over level kernels, whole solves of 1, 2,
+//     3, 4, 6, 8, 12 and 40 iterations, binary64 and binary32:
+//       48^3   0.95 0.88 0.84 0.82 0.80 0.78 0.75 0.72   0.95 0.91 0.88 0.86 0.83 0.82 0.76 0.71
+//       64^3   1.04 0.92 0.89 0.84 0.80 0.78 0.74 0.70   1.01 0.93 0.90 0.87 0.82 0.81 0.74 0.68
+//       116^3  1.07 0.97 0.91 0.89 0.86 0.84 0.81 0.77   1.07 0.98 0.94 0.91 0.86 0.84 0.78 0.71
+//       120^3  1.09 1.00 0.95 0.92 0.89 0.87 0.84 0.80   1.10 1.05 1.00 0.98 0.93 0.91 0.85 0.79
+//       128^3  1.11 1.01 0.98 0.94 0.91 0.88 0.86 0.82   1.11 1.06 1.01 0.98 0.95 0.92 0.86 0.80
+//     two tiles a multiprocessor:
+//       131^3  1.15 1.07 1.03 1.00 0.96 0.95 0.92 0.88   1.16 1.11 1.08 1.05 1.02 0.99 0.95 0.90
+//       165^3  1.18 1.12 1.08 1.06 1.03 1.01 0.98 0.95   1.15 1.10 1.08 1.05 1.01 0.99 0.96 0.89
+//   - With more tiles a multiprocessor binary64 gains nothing (three, 176^3:
+//     1.05 at 12 iterations, 1.01 at 40, 0.99 at 80), binary32 up to four (176^3
+//     1.01, 0.98, 0.93 at 8, 12 and 40; 190^3 1.03, 1.00, 0.94; five, 208^3,
+//     1.08, 1.06, 1.02).
+#define TFS_TILE_BLOCK32_ROWS 3072
+#define TFS_TILE_BLOCK64_ROWS 900
+#define TFS_TILE_FROM2_ROWS (1 << 17)
+#define TFS_TILE_FROM4_ROWS 1650000
+template <typename T>
+static bool tiles_pay(const tfs_handle *h, int expected)
+{
+    if (h->dic_tiles == 1) return true;
+    if (dic_block_kind<T>(h) && h->n < (sizeof(T) == 4 ? TFS_TILE_BLOCK32_ROWS : TFS_TILE_BLOCK64_ROWS)) return false;
+    const int a_sm = (tile_count(h->n, h->sm_count) + h->sm_count - 1) / h->sm_count;
+    if (a_sm > (sizeof(T) == 4 ? 4 : 2)) return false;
+    return expected >= (a_sm > 2 ? 12 : a_sm == 2 ? 8 : h->n >= TFS_TILE_FROM4_ROWS ? 4 : h->n >= TFS_TILE_FROM2_ROWS ? 2 : 1);
+}
+
 // The tiled DIC's plan for the current layout in values of T; tiles = 0 where
 // there is none, or the host has no memory for making it.
 template <typename T>
@@ -1134,8 +1170,8 @@ static int upload_tiles(tfs_handle *h, TileStore &S, const TilePlan &P)
     return TFS_OK;
 }
 
-// The plan of arithmetic T, made on the first DIC solve (the topology is
-// fixed, so once per mesh).  A plan that does not exist, does not fit the room
+// The plan of arithmetic T, made on the first DIC solve that sweeps by it (the
+// topology is fixed, so once per mesh).  A plan that does not exist, does not fit the room
 // a server left or cannot be had for want of memory leaves tiles = 0: the
 // level kernels sweep.
 template <typename T>
@@ -1793,7 +1829,8 @@ static int get_graph(tfs_handle *h, int method, int prec, int expected, GraphEnt
         return TFS_OK;
     }
     const int reps = body_iterations(h, method, prec, expected);
-    auto key = [&] { return solve_key(h, method, prec) | (h->no_resident << 12) | ((reps > 1) << 13); };
+    const bool tiled = prec == 2 && (h->precision == TFS_MIXED ? use_tiles<float>(h) : use_tiles<double>(h));
+    auto key = [&] { return solve_key(h, method, prec) | (h->no_resident << 12) | ((reps > 1) << 13) | (tiled << 14); };
     auto it = h->graphs.find(key());
     if (it != h->graphs.end()) { *out = &it->second; return TFS_OK; }
     GraphEntry ge;
@@ -1839,11 +1876,13 @@ int tfs_solve_launch(int method, tfs_handle *h, const double *val, double *x, do
     // It therefore runs through the CG kernels (half the work, same bits);
     // TFS_OPT_BICG = 1 runs the two sequences explicitly.
     const int kmethod = (method == TFS_BICG && !h->bicg_literal) ? TFS_CG : method;
-    h->sweep_tiles = prec == 2 && kmethod != TFS_BICG;   // (the literal BiCG sweeps two vectors, by levels)
+    h->last_key = solve_key(h, kmethod, prec);
+    const int expected = expected_iterations(h, h->last_key, niter);
+    h->sweep_tiles = prec == 2 && kmethod != TFS_BICG &&   // (the literal BiCG sweeps two vectors, by levels)
+                     (h->precision == TFS_MIXED ? tiles_pay<float>(h, expected) : tiles_pay<double>(h, expected));
     if (h->sweep_tiles && (rc = h->precision == TFS_MIXED ? ensure_tiles<float>(h) : ensure_tiles<double>(h))) return rc;
     GraphEntry *ge = nullptr;
-    h->last_key = solve_key(h, kmethod, prec);
-    rc = get_graph(h, kmethod, prec, expected_iterations(h, h->last_key, niter), &ge);
+    rc = get_graph(h, kmethod, prec, expected, &ge);
     if (rc) return rc;
     h->last_graph = ge;
     cudaStream_t s = h->stream;
@@ -2063,7 +2102,8 @@ static int vec_out(tfs_handle *h, const double *src, double *host)
 // values in the arithmetic that is going to sweep.
 static int form_prec(tfs_handle *h, int prec, bool sweeps, int mode = TFS_FP64)
 {
-    h->sweep_tiles = prec == 2 && sweeps;
+    h->sweep_tiles = prec == 2 && sweeps &&
+                     (mode == TFS_MIXED ? tiles_pay<float>(h, INT32_MAX) : tiles_pay<double>(h, INT32_MAX));
     if (h->sweep_tiles) {
         int rc = mode == TFS_FP64 ? ensure_tiles<double>(h) : ensure_tiles<float>(h);
         if (rc) return rc;

@@ -154,7 +154,7 @@ struct tfs_handle {
     int eager = 0;                     // TFS_OPT_LAUNCH: 1 launch kernels from a host loop, no CUDA graph
     int bicg_literal = 0;              // TFS_OPT_BICG: 1 BiCG runs its shadow sequence explicitly
     int dic_block = 1;                 // TFS_OPT_DIC_BLOCK: 1 one-block DIC where the vector and two slots of the widest level fit
-    int dic_tiles = 1;                 // TFS_OPT_DIC_TILES: 1 tiled DIC sweeps where the numbering allows
+    int dic_tiles = 2;                 // TFS_OPT_DIC_TILES: 1 tiled DIC sweeps where the numbering allows, 2 and they pay
     bool sweep_tiles = false;          // the call at hand sweeps one vector, tile by tile where it can
     std::shared_ptr<tfs::TilePartition> tile_part;   // of the plan made last, for the other arithmetic's
     TileStore *tiles[2] = {nullptr, nullptr};   // binary32, binary64 plan of the current layout (null: not made yet)

@@ -45,13 +45,13 @@ def _solve(sol, s, method, limit):
 def test_solves_that_end_inside_a_body(kind, shape, mode, gpu):
     s = system(kind, *shape)
     method = TFS_CG if kind == POISSON else TFS_CGS
-    limits = [1, 2, 3, 4, 5, 6, 7, 9]
+    limits = [1, 2, 3, 5, 13, 14, 15, 16, 17]     # singly, then in bodies of four
     with Solver(s.matrix(), precision=mode, options={TFS_OPT_DIC_TILES: 0}) as sol:
         want = [_solve(sol, s, method, n) for n in limits]
 
     def run(_):
         out = []
-        with Solver(s.matrix(), precision=mode) as sol:
+        with Solver(s.matrix(), precision=mode, options={TFS_OPT_DIC_TILES: 1}) as sol:
             for _ in range(4):
                 out.append([_solve(sol, s, method, n) for n in limits])
             assert sol.stats()["dic_tiles"] > 0
