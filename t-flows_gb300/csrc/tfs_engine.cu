@@ -34,6 +34,7 @@ using namespace tfs;
 struct TileStore {
     int tiles = 0;                       // 0: no plan to be had, the level kernels sweep
     int max_slots = 0, max_rounds = 0, max_lists = 0, ring_bytes = 0, smem_bytes = 0;
+    int64_t bytes = 0;                   // on the device
     struct Dir {
         TileRound *rounds = nullptr;
         int *tile_round = nullptr, *vbeg = nullptr;
@@ -565,6 +566,7 @@ static void free_tiles(tfs_handle *h)
     for (TileStore *&S : h->tiles) {
         if (!S) continue;
         free_tiles(*S);
+        h->device_bytes -= S->bytes;
         delete S;
         S = nullptr;
     }
@@ -1102,12 +1104,14 @@ static bool tiles_pay(const tfs_handle *h, int expected)
 // The tiled DIC's plan for the current layout in values of T; tiles = 0 where
 // there is none, or the host has no memory for making it.
 template <typename T>
-static TilePlan make_tiles(tfs_handle *h, int optin)
+static TilePlan make_tiles(tfs_handle *h, int most_threads)
 {
     TilePlan P;
+    int optin = 0;
+    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device) != cudaSuccess) return P;
     try {
         if (!h->tile_part) h->tile_part = std::make_shared<TilePartition>();
-        const int threads = std::max(1, std::min(16, (int)std::thread::hardware_concurrency()));
+        const int threads = std::max(1, std::min(most_threads, (int)std::thread::hardware_concurrency()));
         std::vector<int> internal(h->n);
         for (int k = 0; k < h->n_int; k++)
             if (h->perm_host[k] >= 0) internal[h->perm_host[k]] = k;
@@ -1120,11 +1124,21 @@ static TilePlan make_tiles(tfs_handle *h, int optin)
     return P;
 }
 
-// Copies a plan to the device.  Device memory that is not to be had is no
-// error: what was taken is given back, and the level kernels, which need none
-// of it, sweep.
-static int upload_tiles(tfs_handle *h, TileStore &S, const TilePlan &P)
+// Copies a plan of arithmetic T to the device.  Device memory that is not to be
+// had is no error: what was taken is given back, and the level kernels, which
+// need none of it, sweep.
+template <typename T>
+static int upload_tiles(tfs_handle *h, const TilePlan &P)
 {
+    TileStore *&kept = h->tiles[sizeof(T) == 8];
+    if (!kept) kept = new TileStore;
+    TileStore &S = *kept;
+    if (!P.tiles) return TFS_OK;
+    // (the kernels' limit, not this plan's need: other handles launch them too)
+    int optin = 0;
+    CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
+    CK(cudaFuncSetAttribute(k_dic_tile<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+    CK(cudaFuncSetAttribute(k_dic_tile<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     cudaStream_t s = h->stream;
     const int64_t before = h->device_bytes;
     bool full = false;
@@ -1166,27 +1180,20 @@ static int upload_tiles(tfs_handle *h, TileStore &S, const TilePlan &P)
     S.ring_bytes = P.ring_bytes;
     S.smem_bytes = P.smem_bytes;
     S.tiles = P.tiles;
+    S.bytes = h->device_bytes - before;
     h->stats.device_bytes = h->device_bytes;
     return TFS_OK;
 }
 
 // The plan of arithmetic T, made on the first DIC solve that sweeps by it (the
-// topology is fixed, so once per mesh).  A plan that does not exist, does not fit the room
-// a server left or cannot be had for want of memory leaves tiles = 0: the
-// level kernels sweep.
+// topology is fixed, so once per mesh).  A plan that does not exist or cannot
+// be had for want of memory leaves tiles = 0: the level kernels sweep.  A
+// server makes its handles' plans beside the solves.
 template <typename T>
 static int ensure_tiles(tfs_handle *h)
 {
-    TileStore *&S = h->tiles[sizeof(T) == 8];
-    if (!tiles_allowed<T>(h) || S) return TFS_OK;
-    int optin = 0;
-    CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
-    CK(cudaFuncSetAttribute(k_dic_tile<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-    CK(cudaFuncSetAttribute(k_dic_tile<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-    const TilePlan P = make_tiles<T>(h, optin);
-    S = new TileStore;
-    if (!P.tiles || P.bytes() > h->tile_room) return TFS_OK;
-    return upload_tiles(h, *S, P);
+    if (h->served || !tiles_allowed<T>(h) || h->tiles[sizeof(T) == 8]) return TFS_OK;
+    return upload_tiles<T>(h, make_tiles<T>(h, 16));
 }
 
 // Whether the sweeps of arithmetic T run tile by tile: they may, the entry point
@@ -1205,6 +1212,39 @@ static TileDev tile_dev(const tfs_handle *h, int d)
     const TileStore::Dir &E = S.dir[d];
     return TileDev{E.rounds, E.tile_round, E.rows, E.vbeg, E.packed, E.tile_list, E.lists, E.list_row, E.list_slot,
                    S.max_slots, S.max_rounds, S.max_lists, S.ring_bytes};
+}
+
+// A server's side of the plans: whether the solve launched last would have swept
+// by a plan that has not been made, the device bytes that it takes at least,
+// the plan (host work only; the handle may solve meanwhile), and its arrival
+// and removal on a handle that is idle.
+bool tfs_tiles_missing(const tfs_handle *h)
+{
+    if (!h->sweep_tiles || h->tiles[h->precision == TFS_FP64]) return false;
+    return h->precision == TFS_FP64 ? tiles_allowed<double>(h) : tiles_allowed<float>(h);
+}
+int64_t tfs_tiles_least_bytes(const tfs_handle *h, int mode)
+{
+    // every row and every off-diagonal entry once, both directions
+    const int64_t ts = mode == TFS_FP64 ? 8 : 4;
+    return 2 * (int64_t)h->n * (15 + ts) + ((int64_t)h->nnz - h->n) * (2 + ts);
+}
+TilePlan tfs_tiles_make(tfs_handle *h, int mode)
+{
+    return mode == TFS_FP64 ? make_tiles<double>(h, 8) : make_tiles<float>(h, 8);
+}
+int tfs_tiles_install(tfs_handle *h, int mode, const TilePlan &P)
+{
+    CK(cudaSetDevice(h->device));
+    return mode == TFS_FP64 ? upload_tiles<double>(h, P) : upload_tiles<float>(h, P);
+}
+bool tfs_tiles_drop(tfs_handle *h)
+{
+    const int64_t before = h->device_bytes;
+    cudaSetDevice(h->device);
+    drop_graphs(h);
+    free_tiles(h);
+    return h->device_bytes < before;
 }
 
 // D and the values of both directions into sweep order, after the factor is

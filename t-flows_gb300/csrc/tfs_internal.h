@@ -112,6 +112,7 @@ struct Vec32 {
 
 struct FaceMap;   // tfs_assemble.cu
 struct TileStore; // tfs_engine.cu: the tiled DIC's plan on the device
+namespace tfs { struct TilePlan; }   // tfs_dic_tiles_plan.h: and on the host
 namespace tfs { struct TilePartition; }   // tfs_dic_tiles_plan.h
 
 struct GraphEntry {
@@ -158,7 +159,6 @@ struct tfs_handle {
     bool sweep_tiles = false;          // the call at hand sweeps one vector, tile by tile where it can
     std::shared_ptr<tfs::TilePartition> tile_part;   // of the plan made last, for the other arithmetic's
     TileStore *tiles[2] = {nullptr, nullptr};   // binary32, binary64 plan of the current layout (null: not made yet)
-    int64_t tile_room = INT64_MAX;     // device bytes the plan may take (a server's budget)
     bool served = false;               // a server's: other requests' kernels share the multiprocessors
     int tiles_used = 0;                // tiles of the last DIC application launched (0: none)
     unsigned long long dicb_diag_ns = 0;   // tfs_diag_dic_timeout
@@ -222,6 +222,12 @@ int tfs_solve_launch(int method, tfs_handle *h, const double *val, double *x, do
                      int32_t prec, int32_t niter, double tol, bool device_ptrs,
                      const double *b_in = nullptr, int x0_zero = 0);
 int tfs_solve_collect(tfs_handle *h, int32_t *niter, double *ini_res, double *fin_res);
+// The tiled DIC's plans of a served handle (tfs_engine.cu).
+bool tfs_tiles_missing(const tfs_handle *h);
+int64_t tfs_tiles_least_bytes(const tfs_handle *h, int mode);
+tfs::TilePlan tfs_tiles_make(tfs_handle *h, int mode);
+int tfs_tiles_install(tfs_handle *h, int mode, const tfs::TilePlan &P);
+bool tfs_tiles_drop(tfs_handle *h);
 // Device bytes a topology will hold once its layout is built (estimate).
 int64_t tfs_estimate_bytes(int32_t n, int32_t nnz);
 // tfs_assemble.cu

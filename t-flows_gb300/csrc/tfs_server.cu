@@ -12,6 +12,13 @@
 // at a time (a handle is not re-entrant); requests of one system are served
 // in arrival order.  Results do not depend on what else is running: each
 // solve has its own handle state and fixed-order reductions.
+//
+// Tile plans of the DIC sweeps (tfs_dic_tiles_plan.h: up to a second of host
+// work on two million rows, a fifth of the system's device memory and more) are
+// an option, and never cost a request: a system's DIC requests go by the level
+// kernels, to the same bits, until a second thread has made its plan, without
+// the lock; it takes only room that no system added so far needs, and plans go
+// before any system is evicted.
 #include <algorithm>
 #include <chrono>
 #include <condition_variable>
@@ -22,6 +29,7 @@
 #include <thread>
 #include <vector>
 
+#include "tfs_dic_tiles_plan.h"
 #include "tfs_internal.h"
 
 namespace {
@@ -53,7 +61,16 @@ struct System {
     tfs_handle *h = nullptr;
     int64_t bytes = 0;
     bool busy = false;
+    bool planning = false;         // its plan is being made: the handle stays
+    bool hold = false;             // the plan is ready: no request starts until it is on the device
+    int64_t plan_bytes[2] = {0, 0};   // by arithmetic: what the plan takes, once known
+    bool plan_none[2] = {false, false};   // there is none, or no memory for it
     clk::time_point last_used;
+};
+
+struct PlanJob {
+    System *sy;
+    int mode;
 };
 
 }  // namespace
@@ -63,8 +80,9 @@ struct tfs_server {
     int64_t budget = 0, resident = 0;
     int max_inflight = 8;
     std::mutex mu;
-    std::condition_variable cv_work, cv_done;
-    std::thread worker;
+    std::condition_variable cv_work, cv_done, cv_plan;
+    std::thread worker, planner;
+    std::deque<PlanJob> plans;
     bool stop = false;
     std::deque<Request *> queue;
     std::vector<Request *> running;
@@ -91,24 +109,112 @@ static void release_system(tfs_server *S, System &sy)
     sy.h = nullptr;
     S->resident -= sy.bytes;
     sy.bytes = 0;
+    sy.plan_none[0] = sy.plan_none[1] = false;
     S->stats.evictions++;
 }
 
-// Make room for `need` bytes by evicting idle systems, least recently used
-// first.  Caller holds the lock.
+// Room that no system added so far needs.  Caller holds the lock.
+static int64_t spare_room(const tfs_server *S)
+{
+    int64_t room = S->budget;
+    for (const auto &kv : S->systems) room -= kv.second.h ? kv.second.bytes : tfs_estimate_bytes(kv.second.n, kv.second.nnz);
+    return room;
+}
+
+// The plans of the idle systems, least recently used first, until `need` bytes
+// fit.  Caller holds the lock.
+static void drop_plans(tfs_server *S, int64_t need)
+{
+    std::vector<System *> idle;
+    for (auto &kv : S->systems)
+        if (kv.second.h && !kv.second.busy && !kv.second.planning) idle.push_back(&kv.second);
+    std::sort(idle.begin(), idle.end(), [](const System *a, const System *b) { return a->last_used < b->last_used; });
+    for (System *sy : idle) {
+        if (S->resident + need <= S->budget) return;
+        if (!tfs_tiles_drop(sy->h)) continue;
+        S->resident += sy->h->device_bytes - sy->bytes;
+        sy->bytes = sy->h->device_bytes;
+    }
+}
+
+// Make room for `need` bytes by giving up plans, then by evicting idle systems,
+// least recently used first.  Caller holds the lock.
 static bool make_room(tfs_server *S, int64_t need, int64_t keep)
 {
+    if (S->resident + need > S->budget) drop_plans(S, need);
     while (S->resident + need > S->budget) {
         System *victim = nullptr;
         for (auto &kv : S->systems) {
             System &sy = kv.second;
-            if (!sy.h || sy.busy || kv.first == keep) continue;
+            if (!sy.h || sy.busy || sy.planning || kv.first == keep) continue;
             if (!victim || sy.last_used < victim->last_used) victim = &sy;
         }
         if (!victim) return false;
         release_system(S, *victim);
     }
     return true;
+}
+
+static void planner_main(tfs_server *S);
+
+// After a launch: a plan that the system's DIC requests would sweep by, if it
+// fits.  Caller holds the lock.
+static void ask_for_plan(tfs_server *S, System &sy)
+{
+    if (sy.planning || !tfs_tiles_missing(sy.h)) return;
+    const int mode = sy.h->precision, k = mode == TFS_FP64;
+    if (sy.plan_none[k] || std::max(sy.plan_bytes[k], tfs_tiles_least_bytes(sy.h, mode)) > spare_room(S)) return;
+    try {
+        S->plans.push_back(PlanJob{&sy, mode});
+        if (!S->planner.joinable()) S->planner = std::thread(planner_main, S);
+    } catch (const std::exception &) {   // no memory, no thread: no plans
+        if (!S->planner.joinable()) S->plans.clear();
+        sy.plan_none[k] = true;
+        return;
+    }
+    sy.planning = true;
+    S->cv_plan.notify_all();
+}
+
+// Makes the plans asked for, one at a time, and puts each on the device when
+// its system is idle and the room is still there.
+static void planner_main(tfs_server *S)
+{
+    cudaSetDevice(S->device);
+    std::unique_lock<std::mutex> lk(S->mu);
+    for (;;) {
+        S->cv_plan.wait(lk, [&] { return S->stop || !S->plans.empty(); });
+        if (S->stop) return;
+        System &sy = *S->plans.front().sy;
+        const int mode = S->plans.front().mode, k = mode == TFS_FP64;
+        S->plans.pop_front();
+        lk.unlock();
+        tfs::TilePlan P = tfs_tiles_make(sy.h, mode);
+        const int64_t bytes = P.bytes();
+        lk.lock();
+        if (P.tiles) sy.plan_bytes[k] = bytes;
+        else sy.plan_none[k] = true;
+        if (P.tiles && bytes <= spare_room(S)) {
+            sy.hold = true;
+            S->cv_plan.wait(lk, [&] { return S->stop || !sy.busy; });
+            if (!S->stop && bytes <= spare_room(S)) {
+                sy.busy = true;
+                sy.bytes += bytes;
+                S->resident += bytes;
+                lk.unlock();
+                const int rc = tfs_tiles_install(sy.h, mode, P);
+                P = tfs::TilePlan();
+                lk.lock();
+                sy.busy = false;
+                if (rc || sy.h->device_bytes < sy.bytes) sy.plan_none[k] = true;   // no device memory
+                S->resident += sy.h->device_bytes - sy.bytes;
+                sy.bytes = sy.h->device_bytes;
+            }
+            sy.hold = false;
+        }
+        sy.planning = false;
+        S->cv_work.notify_one();
+    }
 }
 
 // Admit and launch one queued request if its system is idle and resident
@@ -124,7 +230,7 @@ static bool try_start(tfs_server *S, Request *r)
         return true;
     }
     System &sy = it->second;
-    if (sy.busy) return false;
+    if (sy.busy || sy.hold) return false;
     if (!sy.h) {
         int64_t need = tfs_estimate_bytes(sy.n, sy.nnz);
         if (need > S->budget) {
@@ -157,7 +263,6 @@ static bool try_start(tfs_server *S, Request *r)
         S->stats.registrations++;
     }
     tfs_set_precision(sy.h, r->mode);
-    sy.h->tile_room = std::max<int64_t>(0, S->budget - S->resident);   // what a DIC tile plan may take
     r->t_start = clk::now();
     int rc = tfs_solve_launch(r->method, sy.h, r->val, r->x, r->r1, r->prec, r->niter, r->tol, !r->host,
                               r->host ? nullptr : r->b, r->x0_zero);
@@ -170,6 +275,7 @@ static bool try_start(tfs_server *S, Request *r)
     // The layout now exists: account its real size.
     S->resident += sy.h->device_bytes - sy.bytes;
     sy.bytes = sy.h->device_bytes;
+    ask_for_plan(S, sy);
     sy.busy = true;
     sy.last_used = r->t_start;
     r->state = 1;
@@ -191,6 +297,7 @@ static void finish(tfs_server *S, Request *r, System &sy)
     r->t_done = clk::now();
     r->state = 2;
     sy.busy = false;
+    if (sy.hold) S->cv_plan.notify_all();
     sy.last_used = r->t_done;
     S->stats.completed++;
 }
@@ -213,6 +320,7 @@ static void worker_main(tfs_server *S)
                 r->state = 2;
                 r->t_done = clk::now();
                 sy.busy = false;
+                if (sy.hold) S->cv_plan.notify_all();
             } else {
                 finish(S, r, sy);
             }
@@ -269,7 +377,9 @@ extern "C" int tfs_server_destroy(tfs_server *S)
         S->stop = true;
     }
     S->cv_work.notify_all();
+    S->cv_plan.notify_all();
     S->worker.join();
+    if (S->planner.joinable()) S->planner.join();   // (a plan being made is finished first)
     cudaSetDevice(S->device);
     for (auto &kv : S->systems)
         if (kv.second.h) tfs_release(kv.second.h);
