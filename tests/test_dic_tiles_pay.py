@@ -28,7 +28,9 @@ LINES = [((14, 15, 14), TFS_MIXED, {1: 0, 40: 0}), ((15, 15, 14), TFS_MIXED, {1:
          ((10, 9, 9), TFS_FP64, {1: 0, 40: 0}), ((10, 10, 9), TFS_FP64, {1: 1, 40: 1}),
          ((51, 51, 50), TFS_FP64, {1: 1, 2: 1}), ((51, 51, 51), TFS_FP64, {1: 0, 2: 1}),
          ((119, 119, 117), TFS_MIXED, {3: 0, 4: 1}), ((131, 131, 130), TFS_MIXED, {7: 0, 8: 1}),
-         ((131, 131, 130), TFS_FP64, {7: 0, 8: 1})]
+         ((131, 131, 130), TFS_FP64, {7: 0, 8: 1}),
+         # one tile a multiprocessor by its rows, but in binary64 they do not fit: two
+         ((129, 129, 129), TFS_FP64, {3: 0, 4: 1})]
 
 
 @pytest.mark.parametrize("shape,mode,asked", LINES)

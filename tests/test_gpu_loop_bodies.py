@@ -8,7 +8,7 @@ import pytest
 
 from helpers import system
 from tflows import TFS_BICG, TFS_CG, TFS_CGS, TFS_FP64, TFS_MIXED, Solver
-from tflows.lib import TFS_OPT_BICG, TFS_OPT_LAUNCH
+from tflows.lib import TFS_OPT_BICG, TFS_OPT_DIC_TILES, TFS_OPT_LAUNCH
 from tflows.synth import CONVDIFF, POISSON
 
 pytestmark = pytest.mark.gpu
@@ -52,7 +52,8 @@ def test_kernel_launches_count_whole_bodies(mode, prec, gpu):
         it = _solve(sol, s, TFS_CG, prec, limit, rel)[2][2]
         return it, sol.stats()["kernel_launches"]
 
-    with Solver(s.matrix(), precision=mode) as sol:
+    # (tiles whatever the limit: without iterations the level kernels are the default)
+    with Solver(s.matrix(), precision=mode, options={TFS_OPT_DIC_TILES: 1}) as sol:
         assert count(sol, 0, 1e-30)[0] == 0
         around = sol.stats()["kernel_launches"]
         one = count(sol, 1, 1e-30)[1] - around
