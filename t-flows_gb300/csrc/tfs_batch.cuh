@@ -61,23 +61,34 @@ struct BatchCtl {
 };
 
 #define TFS_BATCH_MAX_TPB 512
-// CTAs of 512 threads an SM is to hold: one (128 registers, no spilling) or,
-// for batches that ask for more CTAs than TFS_BATCH_ROOMY (binary64:
-// TFS_BATCH_CROWDED) an SM, two (64 registers, some spilling).  Measured, one / two, ms: 24 systems of
-// 5k to 91k cells mixed 16 x 512 10.6 / 10.2, 8 x 512 9.6 / 14.0; 96 systems
-// of up to 500k cells mixed 16 x 512 235 / 197, 8 x 512 221 / 215; binary64
-// 24 systems 27.7 / 31.7 and 39.9 / 43.6, 96 systems 608 / 583 and 539 / 569.
-// (Three, as long as the whole system's pointers and every thread's copy of
-// the solve's scalars were spilled: 20.8 and 21.5, 249 and 353; binary64 45.8
-// and 48.7, 622 and 751.)
-// Binary64 by CTAs asked for per SM, one / two / three, ms: 3.4 (64 systems of
-// up to 500k cells, 8 x 512) 366 / 490 / 655, 6.7 (16 x 512) 337 / 341 / 478,
-// 13.5 (256 systems, 8 x 512) 1267 / 1043 / 1127, 27 (16 x 512) 1439 / 1375 /
-// 1418.  Binary32 with DIC, whose level barriers leave most to wait for, two /
-// three: 5.1 (96 systems, 8 x 512, 60 iterations) 87 / 105, 8.4 (160 systems)
-// 132 / 120.
+// CTAs of 512 threads an SM is to hold: one (128 registers, no spilling), two
+// (64, some spilling) or three (42).  More hold more systems at once, each
+// slower for it.  `asked`: the CTAs of the whole batch, in 512 threads, for each
+// SM; `work`: the same with every system counted by its rows over the largest's,
+// which is what there is to do beside the largest.  Measured, one / two / three,
+// ms, 60 iterations (systems log-uniform in a range of cells):
+//   DIC, whose level barriers leave most to wait for: two as soon as one does not
+//   hold the batch, three where two do not, unless the rows of a thread are many
+//   and the largest system dominates:
+//     mixed    24 of 2k to 30k, 8 x 512 (asked 1.3)   10.6   7.1   7.6
+//              64 of 2k to 30k, 8 x 512 (3.4)         26.7  12.7  12.0
+//             110 of 2k to 30k, 8 x 512 (5.8)         43.0  22.7  19.5
+//              64 of 20k to 200k, 8 x 512 (3.4; work 1.3)  61.1  37.9  42.8
+//             100 of 20k to 200k, 8 x 512 (5.3; work 2.1)  91.6  56.3  52.8
+//     binary64 64 of 2k to 30k, 8 x 512                35.8  19.3  17.7
+//             110 of 2k to 30k, 8 x 512                58.3  32.2  28.9
+//   binary64 without DIC: two where the work asked is more than one holds:
+//             110 of 2k to 30k, 8 x 512 (work 2.0)     12.0   8.8   8.7
+//              64 of 20k to 200k, 8 x 512 (1.3)        29.7  26.2  32.9
+//              64 of 5k to 500k, 8 x 512 (0.7)         366   490   655
+//              64 of 5k to 500k, 16 x 512 (1.5)        337   341   478
+//             256 of 5k to 500k, 8 x 512 (2.9)        1267  1043  1127
+//   mixed without DIC: two past TFS_BATCH_ROOMY CTAs an SM:
+//              24 of 5k to 91k, 8 x 512               9.6  14.0
+//              96 of up to 500k, 16 x 512             235   197
 #define TFS_BATCH_ROOMY 3
-#define TFS_BATCH_CROWDED 8
+#define TFS_BATCH_WIDE_ROWS 16      // rows of a thread from which the largest system's own time counts
+#define TFS_BATCH_WIDE_WORK 1.6
 
 // Sum of NV values over the cluster: block sum, one partial per CTA in
 // shared memory, cluster barrier, the C partials added in rank order.  The

@@ -2604,14 +2604,31 @@ extern "C" int tfs_batch_configure(tfs_batch *b, int cluster_size, int threads_p
     return TFS_OK;
 }
 
+// CTAs of 512 threads a multiprocessor is to hold (tfs_batch.cuh).
+template <int METHOD, typename VT>
+static int batch_per_sm(const tfs_batch *b)
+{
+    const double sms = b->hs[0]->sm_count, threads = (double)b->cluster * b->tpb;
+    if (METHOD != 2 && sizeof(VT) == 4) return (double)b->n * b->cluster > TFS_BATCH_ROOMY * sms ? 2 : 1;
+    double rows = 0.0, largest = 1.0;
+    for (const tfs_handle *h : b->hs) {
+        rows += h->n;
+        largest = std::max(largest, (double)h->n);
+    }
+    const double a_system = threads / (TFS_BATCH_MAX_TPB * sms);   // CTAs of 512 threads a multiprocessor
+    const double asked = b->n * a_system, work = rows / largest * a_system;
+    if (METHOD != 2) return work > 1.0 ? 2 : 1;
+    if (asked <= 1.0) return 1;
+    return asked <= 2.0 || (largest > TFS_BATCH_WIDE_ROWS * threads && work <= TFS_BATCH_WIDE_WORK) ? 2 : 3;
+}
+
 template <int METHOD, typename VT>
 static int launch_batch_kernel(tfs_batch *b)
 {
-    const int64_t asked = (int64_t)b->n * b->cluster, sms = b->hs[0]->sm_count;
-    auto kernel = asked > (sizeof(VT) == 4 ? TFS_BATCH_ROOMY : TFS_BATCH_CROWDED) * sms ? k_batch<METHOD, VT, 2>
-                                                                                        : k_batch<METHOD, VT, 1>;
-    if constexpr (METHOD == 2 && sizeof(VT) == 4)
-        if (asked > TFS_BATCH_CROWDED * sms) kernel = k_batch<METHOD, VT, 3>;
+    const int per_sm = batch_per_sm<METHOD, VT>(b);
+    auto kernel = per_sm == 1 ? k_batch<METHOD, VT, 1> : k_batch<METHOD, VT, 2>;
+    if constexpr (METHOD == 2)
+        if (per_sm == 3) kernel = k_batch<METHOD, VT, 3>;
     if (b->cluster > 8) CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
