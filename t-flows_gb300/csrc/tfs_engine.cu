@@ -1588,6 +1588,16 @@ static K *step_width(int chunks, int grid, K *one, K *two, K *four)
 }
 #define TFS_STEPS(kernel, arg) step_width(nc, G, kernel<arg, 1>, kernel<arg, 2>, kernel<arg, 4>)
 
+// k_cg_update for the chunks, and the blocks a multiprocessor is to hold.
+#define TFS_UPDATE_ONE_WAVE 5
+template <bool FUSED>
+static auto cg_update_kernel(int chunks, int grid, int sms)
+{
+    return step_width(chunks, grid,
+                      chunks <= TFS_UPDATE_ONE_WAVE * sms ? k_cg_update<FUSED, 1, 4> : k_cg_update<FUSED, 1, 8>,
+                      k_cg_update<FUSED, 2, 6>, k_cg_update<FUSED, 4, 4>);
+}
+
 static int launch_body(tfs_handle *h, cudaStream_t s, int method, int prec,
                        cudaGraphConditionalHandle cond, int *count)
 {
@@ -1603,7 +1613,7 @@ static int launch_body(tfs_handle *h, cudaStream_t s, int method, int prec,
             if ((rc = launch_sweeps<double>(h, s, 1, V.r, nullptr, V.y, nullptr, V.z, nullptr, count, true))) return rc;
             launch_ex(pv, TFS_STEPS(k_cg_p, true), G, T, s, nc, V, (const DevState *)h->st);
             launch_spmv_pq(h, s, false, pv, use_tiles<double>(h));
-            launch_ex(pv, TFS_STEPS(k_cg_update, false), G, T, s, nc, V, h->st, h->part, cond, l0);
+            launch_ex(pv, cg_update_kernel<false>(nc, G, h->sm_count), G, T, s, nc, V, h->st, h->part, cond, l0);
             *count += 3;
         } else if (prec == 2) {
             const bool pv = h->use_pdl && h->pdl_vec;
@@ -1611,13 +1621,13 @@ static int launch_body(tfs_handle *h, cudaStream_t s, int method, int prec,
             launch_ex(pv, TFS_STEPS(k_dot_rho, 0), G, T, s, nc, V, h->st, h->part);
             launch_ex(pv, TFS_STEPS(k_cg_p, true), G, T, s, nc, V, (const DevState *)h->st);
             launch_spmv_pq(h, s, false, pv, use_tiles<double>(h));
-            launch_ex(pv, TFS_STEPS(k_cg_update, false), G, T, s, nc, V, h->st, h->part, cond, 0);
+            launch_ex(pv, cg_update_kernel<false>(nc, G, h->sm_count), G, T, s, nc, V, h->st, h->part, cond, 0);
             *count += 4;
         } else {
             const bool pv = h->use_pdl && h->pdl_vec;
             launch_ex(pv, TFS_STEPS(k_cg_p, true), G, T, s, nc, V, (const DevState *)h->st);
             launch_spmv_pq(h, s, false, pv);
-            launch_ex(pv, TFS_STEPS(k_cg_update, true), G, T, s, nc, V, h->st, h->part, cond, 0);
+            launch_ex(pv, cg_update_kernel<true>(nc, G, h->sm_count), G, T, s, nc, V, h->st, h->part, cond, 0);
             *count += 3;
         }
     } else if (method == TFS_BICG) {

@@ -1161,13 +1161,15 @@ k_spmv_pq(SellDev A, const double *__restrict__ val, const double *__restrict__ 
 // eight an SM is then two full waves, not the three, the last one short, of
 // the 73 to 78 registers the compiler takes freely (a 128^3 iteration,
 // diagonal 168 -> 158 us, DIC 293 -> 285; capped for eight blocks, with
-// spills, 171 and 297).  Grids of one chunk a block (W = 1) run eight blocks
-// an SM, one wave.  With that, the packed block sums and no rows that a step
-// does not have, 12 us instead of 19 at 64^3 from cold caches; a 64^3
-// iteration, diagonal 45.1 -> 37.1 us, DIC 89.5 -> 78.6, a 128^3 one 158 ->
+// spills, 171 and 297).  Grids of one chunk a block (W = 1) run four blocks
+// an SM, without spills, up to TFS_UPDATE_ONE_WAVE chunks an SM, and beyond that
+// eight, one wave (40 iterations of a diagonal solve, us, four / eight: 43^3 931
+// / 1175, 52^3 1117 / 1330, 56^3 1423 / 1489, 60^3 1595 / 1571).  With that, the
+// packed block sums and no rows that a step does not have, 12 us instead of 19
+// at 64^3 from cold caches; a 64^3 iteration, diagonal 45.1 -> 37.1 us, DIC 89.5 -> 78.6, a 128^3 one 158 ->
 // 153 and 285 -> 280.
-template <bool FUSED, int W>
-__global__ void __launch_bounds__(TFS_TPB, W == 1 ? 8 : W == 2 ? 6 : 4)
+template <bool FUSED, int W, int PER_SM>
+__global__ void __launch_bounds__(TFS_TPB, PER_SM)
 k_cg_update(int n_chunks, Vec64 V, DevState *st, double *part, cudaGraphConditionalHandle cond,
             int l0_rows = 0)
 {
