@@ -14,8 +14,9 @@ from tflows.synth import POISSON
 pytestmark = pytest.mark.gpu
 
 
-# 309, 750 and 764, 1212 and 1220 chunks, 2436
-@pytest.mark.parametrize("shape", [(43, 43, 42), (58, 58, 57), (58, 58, 58), (68, 68, 67), (68, 68, 68), (86, 86, 84)])
+# 312 chunks; 752 and 764; 1212 and 1232; 2428 and 2456
+@pytest.mark.parametrize("shape", [(43, 43, 43), (58, 58, 57), (58, 58, 58), (68, 68, 67), (68, 68, 68), (86, 86, 84),
+                                   (86, 86, 85)])
 @pytest.mark.parametrize("prec", [1, 2])
 def test_update_against_the_oracle(shape, prec, gpu):
     s = system(POISSON, *shape)
