@@ -183,8 +183,24 @@ extern "C" int tfs_faces_register(tfs_handle *h, int32_t n_faces, const int32_t 
     const int n = h->n;
     // Validate against the registered topology: cell numbers in range, the
     // positions of an interior face inside the rows of c1 and c2 and off the
-    // diagonal, boundary faces with c2 <= 0.
-    std::vector<int> cnt(n + 1, 0);
+    // diagonal, boundary faces with c2 <= 0.  On the way the cells are put in
+    // the order of their first faces, those without one at the end.  (What a
+    // cell needs in one place: its faces are all over the mesh, and each visit
+    // is a miss.)
+    struct Cell {
+        int place = -1, faces = 0;
+    };
+    std::vector<Cell> cells(n);
+    std::vector<int> order;
+    order.reserve(n);
+    auto visit = [&](int c) {
+        Cell &q = cells[c];
+        if (q.place < 0) {
+            q.place = (int)order.size();
+            order.push_back(c);
+        }
+        return &q;
+    };
     for (int s = 0; s < n_faces; s++) {
         const int c1 = faces_c[2 * s], c2 = faces_c[2 * s + 1];
         if (c1 < 1 || c1 > n || c2 > n) {
@@ -198,24 +214,11 @@ extern "C" int tfs_faces_register(tfs_handle *h, int32_t n_faces, const int32_t 
                 tfs_set_error_text("tfs_faces_register: pos does not match the registered topology");
                 return TFS_ERR_ARG;
             }
-            cnt[c2]++;
         }
-        cnt[c1]++;
+        visit(c1 - 1)->faces++;
+        if (c2 > 0) visit(c2 - 1)->faces++;
     }
-    // Cells in the order of their first faces, then the cells without one.
-    std::vector<int> order, place(n, -1);
-    order.reserve(n);
-    auto put = [&](int c) {
-        if (place[c] < 0) {
-            place[c] = (int)order.size();
-            order.push_back(c);
-        }
-    };
-    for (int s = 0; s < n_faces; s++) {
-        put(faces_c[2 * s] - 1);
-        if (faces_c[2 * s + 1] > 0) put(faces_c[2 * s + 1] - 1);
-    }
-    for (int c = 0; c < n; c++) put(c);
+    for (int c = 0; c < n; c++) visit(c);
     const int n_slices = (n + 31) / 32;
     std::vector<int> slice_off(n_slices + 1, 0), begin(n), count(n);
     std::vector<uint32_t> info(n);
@@ -224,9 +227,9 @@ extern "C" int tfs_faces_register(tfs_handle *h, int32_t n_faces, const int32_t 
         int width = 0;
         for (int k = 32 * s; k < std::min(n, 32 * s + 32); k++) {
             const int c = order[k];
-            width = std::max(width, cnt[c + 1]);
+            width = std::max(width, cells[c].faces);
             begin[k] = h->row0[c];
-            count[k] = cnt[c + 1];
+            count[k] = cells[c].faces;
             info[k] = (uint32_t)(h->row0[c + 1] - h->row0[c]) | (uint32_t)(h->dia0[c] - h->row0[c]) << 16;
         }
         slice_off[s] = (int)total;
@@ -237,13 +240,20 @@ extern "C" int tfs_faces_register(tfs_handle *h, int32_t n_faces, const int32_t 
         }
     }
     slice_off[n_slices] = (int)total;
-    std::vector<int> fill(n, 0);
+    // (from here on: the place of the cell's next incidence, its row's start)
+    struct Next {
+        uint32_t at;
+        int row;
+    };
+    std::vector<Next> next(n);
+    for (int k = 0; k < n; k++) next[order[k]] = Next{(uint32_t)(slice_off[k >> 5] + (k & 31)), begin[k]};
     std::vector<uint32_t> code((size_t)total + 1, 0u);
     std::vector<uint16_t> off((size_t)total + 1, 0);
     auto add = [&](int c, uint32_t f, int at) {
-        const size_t e = (size_t)slice_off[place[c] >> 5] + 32 * (size_t)fill[c]++ + (size_t)(place[c] & 31);
-        code[e] = f;
-        off[e] = at < 0 ? kBoundary : (uint16_t)(at - h->row0[c]);
+        Next &q = next[c];
+        code[q.at] = f;
+        off[q.at] = at < 0 ? kBoundary : (uint16_t)(at - q.row);
+        q.at += 32;
     };
     for (int s = 0; s < n_faces; s++) {   // ascending s: each cell's list ends up sorted
         const int c1 = faces_c[2 * s], c2 = faces_c[2 * s + 1];
