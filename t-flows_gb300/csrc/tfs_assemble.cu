@@ -44,7 +44,6 @@ namespace {
 
 constexpr int kTB = 256;
 constexpr int kRow = 8;              // entries of a row held in shared memory
-constexpr int kBatch = 4;            // faces whose coefficients are in flight at once
 constexpr uint16_t kBoundary = 0xffffu;   // entry offset of a boundary face
 
 // The mesh's faces by cell, in the order of the cells' first faces; slices of
@@ -59,8 +58,9 @@ struct FaceMapDev {
     const uint16_t *off;             // offset in the row of the entry the face updates
 };
 
-// The cell's faces on its row `v` (its own memory or shared), diagonal dv.
-template <typename Row>
+// The cell's faces on its row `v` (its own memory or shared), diagonal dv;
+// kBatch faces' coefficients are in flight at once.
+template <int kBatch = 4, typename Row>
 __device__ __forceinline__ double assemble_row(const FaceMapDev &F, Row v, double dv, int e0, int n,
                                                const double *__restrict__ off12, const double *__restrict__ off21,
                                                const double *__restrict__ dia12, const double *__restrict__ dia21)
@@ -103,6 +103,27 @@ __device__ __noinline__ double assemble_long_row(const FaceMapDev &F, double *v,
                                                  const double *dia21)
 {
     return assemble_row(F, v, dv, e0, n, off12, off21, dia12, dia21);
+}
+
+// Cells that come in the order of their rows (a structured numbering): a row a
+// thread, in place and face by face.  The rows of a warp are one run of memory
+// and its coefficients nearly so, so the caches serve a walk along them, and
+// what counts is how many warps walk: 128^3 lexicographic 132 us, with two
+// faces in flight 142 to 153, four 157 to 190; with the rows through shared
+// memory (k_assemble_faces) 197, by cell number with the incidence lists 165.
+__global__ void __launch_bounds__(kTB, 4)
+k_assemble_ordered(FaceMapDev F, const double *__restrict__ off12, const double *__restrict__ off21,
+                   const double *__restrict__ dia12, const double *__restrict__ dia21,
+                   const double *__restrict__ cell, double *val)
+{
+    for (int k = blockIdx.x * kTB + threadIdx.x; k < F.n_cells; k += gridDim.x * kTB) {
+        double *const v = val + __ldg(F.begin + k);
+        const int dia = (int)(__ldg(F.info + k) >> 16), n = __ldg(F.count + k);
+        double dv = assemble_row<1>(F, v, v[dia], __ldg(F.slice_off + (k >> 5)) + (k & 31), n, off12,
+                                    off21, dia12, dia21);
+        if (cell) dv = dv + __ldg(cell + __ldg(F.cell + k));
+        v[dia] = dv;
+    }
 }
 
 __global__ void __launch_bounds__(kTB, 4)
@@ -158,6 +179,7 @@ k_assemble_faces(FaceMapDev F, const double *__restrict__ off12, const double *_
 
 struct FaceMap {
     int n_faces = 0;
+    bool ordered = false;   // most cells come one after the other by number
     int *cell = nullptr, *begin = nullptr, *count = nullptr, *slice_off = nullptr;   // FaceMapDev
     uint32_t *info = nullptr, *code = nullptr;
     uint16_t *off = nullptr;
@@ -265,6 +287,9 @@ extern "C" int tfs_faces_register(tfs_handle *h, int32_t n_faces, const int32_t 
     tfs_faces_free(h);
     FaceMap *F = new FaceMap();
     F->n_faces = n_faces;
+    int follow = 0;
+    for (int k = 1; k < n; k++) follow += order[k] == order[k - 1] + 1;
+    F->ordered = 2 * (int64_t)follow > n;
     h->faces = F;
     auto up = [&](auto **dst, const auto &src) -> cudaError_t {
         const size_t bytes = sizeof(src[0]) * std::max<size_t>(src.size(), 1);
@@ -302,7 +327,8 @@ extern "C" int tfs_assemble_faces_device(tfs_handle *h, const double *d_off12, c
     if (blocks > h->sm_count * 16) blocks = h->sm_count * 16;
     if (blocks < 1) blocks = 1;
     const FaceMapDev D{n, F->cell, F->begin, F->info, F->count, F->slice_off, F->code, F->off};
-    k_assemble_faces<<<blocks, kTB, 0, h->stream>>>(D, d_off12, d_off21, d_dia12, d_dia21, d_cell, d_val);
+    auto kernel = F->ordered ? k_assemble_ordered : k_assemble_faces;
+    kernel<<<blocks, kTB, 0, h->stream>>>(D, d_off12, d_off21, d_dia12, d_dia21, d_cell, d_val);
     e = cudaGetLastError();
     if (e != cudaSuccess) return tfs_engine_error(e, "k_assemble_faces launch");
     return TFS_OK;
