@@ -28,15 +28,18 @@ namespace tfs {
 // SMALL: in binary64 the block sums packed (block_sum_packed; 64^3 17.5 -> 15.9
 // us); in binary32 eight blocks an SM, the whole grid in one wave: with a few
 // chunks a block the kernel waits for its first rows' loads, and twice the
-// warps wait at once (64^3 9.9 -> 7.7 us after tiled sweeps, 8.8 -> 7.2 in a
-// diagonal CG, 90^3 13.3 -> 11.4 there), while a long row loop loses more to
-// the spills of 32 registers (128^3 29.4 -> 32.1).
+// warps wait at once, while a long row loop loses more to the spills of 32
+// registers and a grid that four blocks an SM hold anyway gains nothing.  A
+// mixed solve of 40 iterations, us, without / with, diagonal and DIC: 44^3 757 /
+// 776, 1976 / 1988; 52^3 859 / 876, 2042 / 2062; 64^3 1145 / 999, 2374 / 2187;
+// 90^3 1485 / 1399, 3255 / 3270; 112^3 1979 / 1940, 4398 / 4448; 128^3 2517 /
+// 2557, 5471 / 5596.
 // Minimum resident blocks per SM asked of the compiler (register cap).
 // Unconstrained (1) is kept: on the 128^3 system the binary32 kernel runs
 // at 52 registers (4 blocks per SM) in 31.5 us; capped to 47 or 40
 // registers (5 or 6 blocks, no spills) with the grid at 5 or 6 blocks per
 // SM it took 30.8-30.9 us, inside the run-to-run spread, and capped to 32
-// (8 blocks, with spills) 36.9 us; binary64 73.8 us at 64 registers
+// (8 blocks, with spills) 31.3-32.1 us; binary64 73.8 us at 64 registers
 // against 73.8 us at 48 (5 blocks, small spills).
 #ifndef TFS_PIPE_MINB32
 #define TFS_PIPE_MINB32 1
