@@ -1076,7 +1076,9 @@ static bool tiles_allowed(const tfs_handle *h)
 //     launches cost more than its one.  A solve of 40 iterations, us, one block
 //     / tiles, binary32: 512 rows 1520 / 1631, 1,320 1656 / 1732, 2,940 1781 /
 //     1802, 3,150 1774 / 1734, 4,096 1938 / 1795; binary64: 512 1581 / 1594,
-//     1,320 2159 / 2073, 2,028 2333 / 2148.
+//     1,320 2159 / 2073, 2,028 2333 / 2148.  Rows of more than eight entries
+//     leave the tile kernel's unrolled row: 1,728 rows of up to 11, 20
+//     iterations binary64 1361 / 1497 (8,000 rows, five tiles, 4340 / 1912).
 //   - A solve packs the values first, which comes back after more iterations
 //     the larger the system is.  Tiles over level kernels, whole solves of 1, 2,
 //     3, 4, 6, 8, 12 and 40 iterations, binary64 and binary32:
@@ -1100,7 +1102,8 @@ template <typename T>
 static bool tiles_pay(const tfs_handle *h, int expected)
 {
     if (h->dic_tiles == 1) return true;
-    if (dic_block_kind<T>(h) && h->n < (sizeof(T) == 4 ? TFS_TILE_BLOCK32_ROWS : TFS_TILE_BLOCK64_ROWS)) return false;
+    const int block_rows = sizeof(T) == 4 || h->row_max > 8 ? TFS_TILE_BLOCK32_ROWS : TFS_TILE_BLOCK64_ROWS;
+    if (dic_block_kind<T>(h) && h->n < block_rows) return false;
     const int a_sm = (tile_count(h->n, h->sm_count) + h->sm_count - 1) / h->sm_count;
     if (a_sm > (sizeof(T) == 4 ? 4 : 2)) return false;
     return expected >= (a_sm > 2 ? 12 : a_sm == 2 ? 8 : h->n >= TFS_TILE_FROM4_ROWS ? 4 : h->n >= TFS_TILE_FROM2_ROWS ? 2 : 1);

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 from helpers import system
-from tflows import TFS_CG, TFS_FP64, TFS_MIXED, Solver
+from tflows import TFS_CG, TFS_FP64, TFS_MIXED, Matrix_Type, Solver
 from tflows.lib import TFS_OPT_DIC_TILES
 from tflows.synth import POISSON
 
@@ -69,3 +69,35 @@ def test_short_solves_are_expected_to_be_short_again(gpu):
         assert tiles > 0 and all(np.array_equal(a, b) for a, b in zip(first, again, strict=True))
         _solve(sol, s, 3)                               # ended by its limit: says nothing of the next
         assert _solve(sol, s, 500, 0.99)[1] > 0
+
+
+@pytest.mark.parametrize("mode", [TFS_FP64, TFS_MIXED])
+@pytest.mark.parametrize("n,tiles", [(12, 0), (15, 1)])     # 1,728 and 3,375 rows
+def test_rows_of_more_than_eight_entries(n, tiles, mode, gpu):
+    """A randomly numbered mesh with two diagonal neighbour pairs besides the six
+    faces (rows of up to eleven entries): one block below 3,072 rows in both
+    arithmetics, tiles above, with the level kernels' bits."""
+    num = np.random.default_rng(n).permutation(n ** 3).reshape(n, n, n)
+    rows, cols = [np.arange(n ** 3)], [np.arange(n ** 3)]
+    for dx, dy, dz in ((1, 0, 0), (0, 1, 0), (0, 0, 1), (1, 1, 0), (0, 1, 1)):
+        a, b = num[: n - dx, : n - dy, : n - dz].ravel(), num[dx:, dy:, dz:].ravel()
+        rows += [a, b]
+        cols += [b, a]
+    i, j = np.concatenate(rows), np.concatenate(cols)
+    order = np.lexsort((j, i))
+    i, j = i[order], j[order]
+    deg = np.bincount(i, minlength=n ** 3)
+    val = np.where(i == j, deg[i] - 1 + 0.01, -1.0)
+    row = np.concatenate([[1], 1 + np.cumsum(deg)]).astype(np.int32)
+    A = Matrix_Type(n ** 3, row, (j + 1).astype(np.int32), (np.flatnonzero(i == j) + 1).astype(np.int32), val)
+    b = np.random.default_rng(1).uniform(-1, 1, n ** 3)
+    got = []
+    for option in (0, 1, 2):
+        with Solver(A, precision=mode, options={TFS_OPT_DIC_TILES: option}) as sol:
+            x, r = np.zeros(n ** 3), b.copy()
+            res = sol.solve(TFS_CG, val, x, r, 2, 30, 1e-10)
+            used = sol.stats()["dic_tiles"]
+            assert (used > 0) == (option == 1 or (option == 2 and bool(tiles))), (option, used)
+            got.append((x, r, np.array([res.niter, res.ini_res, res.fin_res])))
+    for other in got[1:]:
+        assert all(np.array_equal(p, q) for p, q in zip(got[0], other, strict=True))
