@@ -383,16 +383,16 @@ k_dic_tile(TileDev P, const T *__restrict__ src, T *__restrict__ dst, DevState *
     }
 }
 
-// D (with its reciprocal, tile_diags) and the values of one direction into the
-// packed rounds (one block per round), from the factor d (internal row order)
-// and the caller's values.
+// D (with its reciprocal, tile_diags) and the values of one direction into round
+// `round` of the packed rounds, from the factor d (internal row order) and the
+// caller's values; a thread a slot.
 template <typename T, int DIR>
-__global__ void __launch_bounds__(TILE_ROWS)
-k_tile_fill(TileDev P, const DevParams *prm, const double *__restrict__ d)
+__device__ __forceinline__ void tile_fill_round(const TileDev &P, int round, const DevParams *prm,
+                                                const double *__restrict__ d)
 {
-    const uint4 c = __ldg(reinterpret_cast<const uint4 *>(P.rounds + blockIdx.x));
+    const uint4 c = __ldg(reinterpret_cast<const uint4 *>(P.rounds + round));
     const int t = threadIdx.x, slices = (int)(c.z >> 16);
-    const size_t slot = (size_t)blockIdx.x * TILE_ROWS + t;
+    const size_t slot = (size_t)round * TILE_ROWS + t;
     const uint32_t w = __ldg(P.rows + slot);
     if ((w & TILE_ROW_MASK) == TILE_NO_ROW) return;
     unsigned char *at = P.packed + 16 * (size_t)c.x;
@@ -405,6 +405,17 @@ k_tile_fill(TileDev P, const DevParams *prm, const double *__restrict__ d)
     const int cnt = (int)((w >> TILE_CNT_SHIFT) & 15u);
     T *tv = td + 32 * slices * tile_diags(DIR, sizeof(T)) + (head & 0xffffu) * 32 + (t & 31);
     for (int j = 0; j < cnt; j++) tv[32 * j] = (T)val[j];
+}
+
+// Both directions' rounds, n0 of them forward; a block a round.  (One launch:
+// a second one was 5 of the 15 us that packing adds to a small solve.)
+template <typename T>
+__global__ void __launch_bounds__(TILE_ROWS)
+k_tile_fill(TileDev P0, TileDev P1, int n0, const DevParams *prm, const double *__restrict__ d)
+{
+    const int b = blockIdx.x;
+    if (b < n0) tile_fill_round<T, 0>(P0, b, prm, d);
+    else tile_fill_round<T, 1>(P1, b - n0, prm, d);
 }
 
 // rho = (r, z) after tiled sweeps, with the terms and the order of

@@ -1262,9 +1262,9 @@ static int launch_tile_fill(tfs_handle *h, cudaStream_t s)
 {
     if (!use_tiles<T>(h)) return 0;
     const TileStore &S = *h->tiles[sizeof(T) == 8];
-    k_tile_fill<T, 0><<<S.dir[0].n_rounds, TILE_ROWS, 0, s>>>(tile_dev<T>(h, 0), h->params, h->v.d);
-    k_tile_fill<T, 1><<<S.dir[1].n_rounds, TILE_ROWS, 0, s>>>(tile_dev<T>(h, 1), h->params, h->v.d);
-    return 2;
+    k_tile_fill<T><<<S.dir[0].n_rounds + S.dir[1].n_rounds, TILE_ROWS, 0, s>>>(tile_dev<T>(h, 0), tile_dev<T>(h, 1),
+                                                                              S.dir[0].n_rounds, h->params, h->v.d);
+    return 1;
 }
 
 // z1 = M^-1 b1 tile by tile (y1: the start values between the sweeps).
