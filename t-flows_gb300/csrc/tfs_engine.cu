@@ -1249,8 +1249,9 @@ int tfs_tiles_install(tfs_handle *h, int mode, const TilePlan &P)
 bool tfs_tiles_drop(tfs_handle *h)
 {
     const int64_t before = h->device_bytes;
+    if (!(h->tiles[0] && h->tiles[0]->tiles) && !(h->tiles[1] && h->tiles[1]->tiles)) return false;
     cudaSetDevice(h->device);
-    drop_graphs(h);
+    drop_graphs(h);   // they hold the plan's addresses
     free_tiles(h);
     return h->device_bytes < before;
 }
